@@ -76,8 +76,33 @@ void drop_graphs(evora_batch* b) {
   b->graphs.clear();
 }
 
-// cap: tubes up to this length are staged in shared memory.
+// Largest shared-memory capacity (cells) that keeps `ctas_per_sm` CTAs.
+int cap_for(const evora_batch* b, int ctas_per_sm) {
+  const size_t per_sm = 227 * 1024;
+  const size_t budget = per_sm / ctas_per_sm - 2048;   // static shared + reserve
+  const size_t per_cell = (size_t)(b->nf + 5) * esize(b);
+  long long cap = (long long)(budget / per_cell) - 4;
+  return (int)std::max(2LL, cap);
+}
+
+// The length of the tube that an average cell-update belongs to (a tube of n
+// cells takes about n steps).
+double work_length(const evora_batch* b) {
+  double n2 = 0.0, n3 = 0.0;
+  for (int v : b->n) {
+    n2 += (double)v * v;
+    n3 += (double)v * v * v;
+  }
+  return n3 / n2;
+}
+
+// cap: tubes up to this length are staged in shared memory.  A single CTA
+// of 512 threads per SM becomes one of 768 where long tubes do most of the
+// work: at 4096 cells 66.9 against 62.1 G cell-updates/s (FP32) and 30.9
+// against 29.4 (FP64), at 8000 cells 48.6 against 40.0; at 2048 cells it
+// loses 1 to 5 %.
 int configure(evora_batch* b, int threads, int cap) {
+  if (threads == 512 && b->nf == 5 && cap >= cap_for(b, 1) && work_length(b) > 2600.0) threads = 768;
   drop_graphs(b);
   BatchPlan& pl = b->plan;
   pl.P = b->P;
@@ -116,13 +141,25 @@ int configure(evora_batch* b, int threads, int cap) {
   return 0;
 }
 
-// Largest shared-memory capacity (cells) that keeps `ctas_per_sm` CTAs.
-int cap_for(const evora_batch* b, int ctas_per_sm) {
-  const size_t per_sm = 227 * 1024;
-  const size_t budget = per_sm / ctas_per_sm - 2048;   // static shared + reserve
-  const size_t per_cell = (size_t)(b->nf + 5) * esize(b);
-  long long cap = (long long)(budget / per_cell) - 4;
-  return (int)std::max(2LL, cap);
+// The default CTA shape by the work-weighted tube length L, from equal tubes
+// of 64 to 8000 cells (G cell-updates/s, FP32 / FP64):
+//   128 threads up to 700 cells (512 cells: 67.8 / 34.5, with 256 60.1 / 28.0),
+//   256 up to 1500 (1024 cells: 69.9 / 33.3, with 512 54.8 / 26.9),
+//   512 above (4096 cells: 64.7 / 30.9, with 256 41.2 / 23.2);
+// as many CTAs per SM as the registers hold, or one that can take any tube in
+// FP64.  With no more than two tubes per SM the longest ones decide, so a tube gets all
+// warps that it has rounds of 30 cells for.
+int configure_default(evora_batch* b) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const double len = work_length(b);
+  const bool f32 = b->precision == EVORA_FP32;
+  if (b->ntubes <= 2 * sms)
+    return configure(b, b->nmax > 480 ? 512 : (b->nmax > 240 ? 256 : 128), cap_for(b, 1));
+  if (len <= 700.0) return configure(b, 128, cap_for(b, f32 ? 6 : 4));
+  if (len <= 1500.0) return configure(b, 256, cap_for(b, f32 ? 3 : 2));
+  return configure(b, 512, cap_for(b, f32 ? 2 : 1));
 }
 
 int upload_order(evora_batch* b) {
@@ -304,7 +341,7 @@ int evora_batch_create(const evora_params* p, int32_t ntubes, const int32_t* n, 
     }
     if (cudaMemcpy(b->tubes, ts.data(), sizeof(TubeState) * ntubes, cudaMemcpyHostToDevice) != cudaSuccess) goto fail;
   }
-  rc = configure(b, 256, cap_for(b, 2));
+  rc = configure_default(b);
   if (rc) {
     free_batch(b);
     return rc;
@@ -486,8 +523,10 @@ int evora_batch_autotune(evora_batch* b, int32_t steps, int32_t* threads_out, in
     int rc = upload_order(b);
     if (rc) return rc;
   }
-  // Save the state and the tube table, time each configuration for `steps`
-  // steps per tube, restore after each trial.
+  // Save the state and the tube table, time each configuration, restore after
+  // each trial.  A trial gives a tube of mean length `steps` steps and the
+  // others in proportion to their length, as a run to a common end time does
+  // (with equal steps per tube the trials favoured short tubes' shapes).
   const size_t qbytes = (size_t)b->nf * b->ntot * esize(b);
   void* save_q = nullptr;
   TubeState* save_t = nullptr;
@@ -511,12 +550,14 @@ int evora_batch_autotune(evora_batch* b, int32_t steps, int32_t* threads_out, in
     for (int ci = 0; ci < 3; ++ci) {
       if (configure(b, cand_threads[ti], cap_for(b, cand_ctas[ci]))) continue;
       b->plan.budget = steps;
+      b->plan.steps_per_cell = (double)steps * b->ntubes / (double)b->ntot;
       CU(cudaEventRecord(e0, b->stream));
       cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
       b->launch(b->plan, b->q, b->stream);
       CU(cudaEventRecord(e1, b->stream));
       CU(cudaEventSynchronize(e1));
       CU(cudaGetLastError());
+      b->plan.steps_per_cell = 0.0;
       float ms = 0.f;
       CU(cudaEventElapsedTime(&ms, e0, e1));
       if (ms < best) {

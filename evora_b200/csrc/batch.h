@@ -32,6 +32,7 @@ struct BatchArgs {
   int* head;              // queue head (reset to 0 before each launch)
   int budget;             // max steps per tube in this launch
   long long quantum;      // if > 0: a tube of n cells runs at most max(1, quantum / n) steps
+  double steps_per_cell;  // if > 0: a tube of n cells runs max(1, steps_per_cell * n) steps (autotune's trials)
   int cap;                // tubes with n <= cap live in shared memory
   int capw;               // cap < n <= capw: w in shared memory, q in the scratch slot
   T* gscratch;            // per-CTA scratch for longer tubes: (NF + 5) * (nmax + 4) each
@@ -53,6 +54,7 @@ struct BatchPlan {
   int* head = nullptr;
   int budget = 1;
   long long quantum = 0;
+  double steps_per_cell = 0.0;
   int cap = 0;
   int capw = 0;        // set with smem: the longest tube whose w fits the shared memory
   void* gscratch = nullptr;

@@ -11,13 +11,18 @@
 //
 // Per step, with the tube in shared memory:
 //   phase 1  primitives of the n cells and the 2+2 ghost cells (index map of
-//            bound, boundary.f90:33-66) into w; per-thread maxima of
-//            |u_d| + a; block reduction; thread 0 forms dt (hydrostep) and
-//            advances t (updatetime);
-//   phase 2  every thread sweeps a contiguous segment of cells like the
-//            reference's pencil loop (muscl.f90:194-215): face states from
-//            the slopes and the predictor, one Riemann solve per interface,
-//            the flux of the previous interface carried, q updated in place.
+//            bound, boundary.f90:33-66) into w, and the block's maximum of
+//            |u_d| + a; every thread forms dt (hydrostep) and advances t
+//            (updatetime) from it;
+//   phase 2  each warp updates 30 consecutive cells at a time (muscl.f90:
+//            194-215): a lane per cell and interface, face states and fluxes
+//            passed on by shuffles (tube_sweep).
+// Bound: instruction issue (57 % of the issue slots at 16 warps per SM, 4 %
+// of HBM).  A lane per interface solves every interface once (1.07 times, with
+// the 2 of 32 lanes that only feed their neighbours); a contiguous segment of
+// cells per thread, as this kernel first had, solved it (n / NT + 1) / (n /
+// NT) times and read w at strides that met in the banks.  4096 tubes of
+// 128-4096 cells, FP32: 245 -> 140 ms; 2048 of them in FP64: 299 -> 155 ms.
 // A tube longer than the shared-memory capacity keeps q in a global scratch
 // slot of its CTA and w in shared memory while w alone fits, else both in
 // the slot (same code, generic pointers).
@@ -29,10 +34,139 @@
 namespace evora {
 namespace EVORA_FNS {
 
+// The maximum over a tube's cells of |u_d| + a as dt = min(cfl min(dx / s,
+// 1e6)): cfl_dt with dx = dy = dz (compparameter's 1D branch), where the
+// smallest of the three quotients is the one by the largest speed.
+__device__ __forceinline__ double cfl_dt1(const HydroParams& P, double smax, unsigned& err) {
+  const double v = fmin2(P.dx / smax, 1e6);
+  const double dt = fmin2(P.cfl * v, 1e99);
+  if (dt <= 0.0) err |= EVORA_ERR_DT;
+  return dt;
+}
+
+// The largest of a non-negative value (no NaN) over a warp, or over red[0..NW)
+// for every lane: values >= 0 order like their bits, which one (FP32) or two
+// (FP64: high words, then the low words of those that have the largest)
+// warp reductions of unsigned words take.
+__device__ __forceinline__ float warp_max_pos(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warp_max_pos(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+// Primitives of the n cells of a tube and its 2 + 2 ghosts (the index map of
+// bound) into w (field-major, stride n + 4); returns this thread's maximum of
+// |u_d| + a over the cells (timestep.f90:40-43), reduced over its warp.  One
+// maximum serves the three axes: a sum of |u_d| and a rounds monotonically,
+// so the largest |u_d| gives the largest sum.
 template <typename T, int NF, int NT>
-__device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int tb, double* red,
-                                         double* bc, unsigned* s_err) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ T tube_primitives(const T* qs, T* w, int n, const HydroParams& P, const Gas<T>& c,
+                                             bool de, unsigned& err) {
+  const int wst = n + 4;
+  T smax = (T)0;
+  for (int i = threadIdx.x; i < wst; i += NT) {
+    bool flip = false;
+    const int g = ghost_map(i - 2, n, P.boundtype, 0, flip);
+    T qv[6], wv[5];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) qv[f] = qs[f * n + g];
+    prim_k(qv, wv, c, P, de, err);
+    if (flip) {
+      wv[1] = -wv[1];
+      wv[2] = -wv[2];
+      wv[3] = -wv[3];
+    }
+#pragma unroll
+    for (int f = 0; f < 5; ++f) w[f * wst + i] = wv[f];
+    if (i >= 2 && i < n + 2) {
+      T a;
+      if constexpr (kFast && sizeof(T) == 8) a = sqrt_fast(c.g * wv[4] * rcp_fast(wv[0]));
+      else a = dsqrt(c.g * wv[4] / wv[0]);
+      const T s = fmax2(fmax2((T)fabs(wv[1]), (T)fabs(wv[2])), (T)fabs(wv[3])) + a;
+      if (s > smax) smax = s;
+    }
+  }
+  return warp_max_pos(smax);
+}
+
+// The update of a tube (muscl.f90:60-69, 194-215) from the primitives in w.
+// A warp takes 32 consecutive cells: every lane forms the face states of
+// its cell, the upper one goes to the next lane by shuffle, a lane solves the
+// interface below its cell, and the flux above comes back by shuffle; the
+// first and last cell only feed their neighbours, so a chunk updates 30
+// cells.  w and q are read and written at consecutive addresses.
+template <typename T, int NF, int NT>
+__device__ __forceinline__ void tube_sweep_opt(T* qs, const T* w, int n, const HydroParams& P, int limiter,
+                                               int solver, bool secondorder, const Gas<T>& c, bool de, double dt,
+                                               unsigned& err) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int wst = n + 4;
+  const T dt2 = (T)(-0.5 * dt);
+  const T dtdx = (T)(dt * P.dxinv);
+  const T dxi = (T)P.dxinv;
+  for (int c0 = 30 * wid; c0 < n; c0 += 30 * (NT / 32)) {
+    const int cc = c0 - 1 + lane;            // this lane's cell, -1 .. n
+    const int wi = (cc < n ? cc : n) + 2;    // lanes past the upper ghost repeat it
+    T wc[5], fm[5], fp[5];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) wc[f] = w[f * wst + wi];
+    if (secondorder) {
+      T s[5], a[5];
+#pragma unroll
+      for (int f = 0; f < 5; ++f) s[f] = slope_k(w[f * wst + wi - 1], wc[f], w[f * wst + wi + 1], limiter);
+      pred_k(wc, s, 1, c.g, kFast ? rcp_fast(wc[0]) : (T)0, a);
+#pragma unroll
+      for (int f = 0; f < 5; ++f) {
+        const T e = dt2 * a[f] * dxi;                  // muscl.f90:68
+        fm[f] = face_minus(wc[f], s[f], e);
+        fp[f] = face_plus(wc[f], s[f], e);
+      }
+    } else {
+#pragma unroll
+      for (int f = 0; f < 5; ++f) fm[f] = fp[f] = wc[f];
+    }
+#pragma unroll
+    for (int f = 0; f < 5; ++f) fp[f] = __shfl_up_sync(0xffffffffu, fp[f], 1);
+    T flo[NF], fhi[NF];
+    unsigned e = 0;
+    riemann_k<T, NF, 1>(fp, fm, flo, solver, c, e);   // interface cc-1/2
+    if (lane > 0 && cc <= n) err |= e;                  // the tube's n + 1 interfaces
+#pragma unroll
+    for (int f = 0; f < NF; ++f) fhi[f] = __shfl_down_sync(0xffffffffu, flo[f], 1);
+    if (lane > 0 && lane < 31 && cc < n) {
+      T qv[6];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) qv[f] = qs[f * n + cc];
+      if (de) {
+        T wd[5];
+        unsigned e2 = 0;
+        prim_k(qv, wd, c, P, de, e2);   // dual-energy resync of q (comp.f90:60-72)
+      }
+#pragma unroll
+      for (int f = 0; f < NF; ++f) qs[f * n + cc] = qv[f] + dtdx * (flo[f] - fhi[f]);
+    }
+  }
+}
+
+// The usual options (minmod, HLLC, second order) as constants, so that their
+// sweep has no branches on them.
+template <typename T, int NF, int NT>
+__device__ __forceinline__ void tube_sweep(T* qs, const T* w, int n, const HydroParams& P, const Gas<T>& c, bool de,
+                                           double dt, unsigned& err) {
+  if (P.limiter == 1 && P.solver == 2 && P.secondorder && !de)
+    tube_sweep_opt<T, NF, NT>(qs, w, n, P, 1, 2, true, c, false, dt, err);
+  else
+    tube_sweep_opt<T, NF, NT>(qs, w, n, P, P.limiter, P.solver, P.secondorder != 0, c, de, dt, err);
+}
+
+template <typename T, int NF, int NT>
+__device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int tb, T* red,
+                                         unsigned* s_err) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   TubeState* ts = A.tubes + tb;
   const int n = ts->n;
   const long long off = ts->offset;
@@ -56,7 +190,6 @@ __device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int
   P.dzinv = 1.0 / P.dz;
   const Gas<T> c = Gas<T>::make(P);
   const bool de = P.dualenergy != 0;
-  const int wst = n + 4;        // w row stride (2 ghosts each side)
   // stage q into qs (field-major, stride n)
   for (int f = 0; f < NF; ++f)
     for (int i = tid; i < n; i += NT) qs[f * n + i] = A.q[(size_t)f * A.ntot + off + i];
@@ -69,128 +202,34 @@ __device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int
     const long long b = A.quantum / n;
     budget = (int)(b < 1 ? 1 : (b < budget ? b : budget));
   }
+  if (A.steps_per_cell > 0.0) budget = max(1, (int)(A.steps_per_cell * n));
   __syncthreads();
   while (steps < budget) {
-    // ---- phase 1: primitives (+ ghosts) and the CFL maxima
-    double m0 = 0.0, m1 = 0.0, m2 = 0.0;
-    for (int i = tid; i < wst; i += NT) {
-      bool flip = false;
-      const int g = ghost_map(i - 2, n, P.boundtype, 0, flip);
-      T qv[6], wv[5];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) qv[f] = qs[f * n + g];
-      prim_k(qv, wv, c, P, de, err);
-      if (flip) {
-        wv[1] = -wv[1];
-        wv[2] = -wv[2];
-        wv[3] = -wv[3];
-      }
-#pragma unroll
-      for (int f = 0; f < 5; ++f) w[f * wst + i] = wv[f];
-      if (i >= 2 && i < n + 2) {
-        // hydrostep speeds (timestep.f90:40-43), reduced in FP64
-        const T a = dsqrt(c.g * wv[4] / wv[0]);
-        const double s0 = (double)(fabs(wv[1]) + a), s1 = (double)(fabs(wv[2]) + a),
-                     s2 = (double)(fabs(wv[3]) + a);
-        if (s0 > m0) m0 = s0;
-        if (s1 > m1) m1 = s1;
-        if (s2 > m2) m2 = s2;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      m0 = fmax2(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-      m1 = fmax2(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-      m2 = fmax2(m2, __shfl_xor_sync(0xffffffffu, m2, o));
-    }
-    const int lane = tid & 31, wid = tid >> 5;
-    if (lane == 0) {
-      red[3 * wid + 0] = m0;
-      red[3 * wid + 1] = m1;
-      red[3 * wid + 2] = m2;
-    }
+    // ---- phase 1: primitives (+ ghosts) and the CFL maximum
+    const T sm = tube_primitives<T, NF, NT>(qs, w, n, P, c, de, err);
+    if (lane == 0) red[wid] = sm;
     if (err) atomicOr(s_err, err);
     __syncthreads();
-    if (tid == 0) {
-      double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-      for (int k = 0; k < NT / 32; ++k) {
-        a0 = fmax2(a0, red[3 * k]);
-        a1 = fmax2(a1, red[3 * k + 1]);
-        a2 = fmax2(a2, red[3 * k + 2]);
-      }
-      unsigned e = *s_err;
-      double d = cfl_dt(P, a0, a1, a2, 1e99, e);
-      int g2 = 1;
-      double tt = t;
-      if (!e) update_time(tend, tt, d, g2);
-      if (!e && g2 && !(tt > t)) e |= EVORA_ERR_DT;   // dt below the resolution of t: no progress
-      bc[0] = d;
-      bc[1] = tt;
-      bc[2] = e ? 1.0 : 0.0;
-      bc[3] = g2;
-      *s_err = e;
+    // every thread forms dt and advances t from the warps' maxima
+    unsigned e = *s_err;
+    const double smax = (double)warp_max_pos(lane < NT / 32 ? red[lane] : (T)0);
+    double d = cfl_dt1(P, smax, e), tt = t;
+    int g2 = 1;
+    if (!e) update_time(tend, tt, d, g2);
+    if (!e && g2 && !(tt > t)) e |= EVORA_ERR_DT;   // dt below the resolution of t: no progress
+    if (e) {                       // an error stops the tube before its update
+      err |= e;
+      break;
     }
-    __syncthreads();
-    if (bc[2] != 0.0) break;       // an error stops the tube before its update
-    dt = bc[0];
-    t = bc[1];
-    go = (int)bc[3];
-    // ---- phase 2: segment sweeps
-    const T dt2 = (T)(-0.5 * dt);
-    const T dtdx = (T)(dt * P.dxinv);
-    const T dxi = (T)P.dxinv;
-    const int seg = (n + NT - 1) / NT;
-    const int i0 = tid * seg;
-    const int i1 = i0 + seg < n ? i0 + seg : n;
-    if (i0 < i1) {
-      T fp_prev[5], flo[NF];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) flo[f] = (T)0;
-      for (int cc = i0 - 1; cc <= i1; ++cc) {
-        const int wi = cc + 2;
-        T wc[5], fm[5], fp[5];
-#pragma unroll
-        for (int f = 0; f < 5; ++f) wc[f] = w[f * wst + wi];
-        if (P.secondorder) {
-          T s[5], a[5];
-#pragma unroll
-          for (int f = 0; f < 5; ++f) s[f] = slope_k(w[f * wst + wi - 1], wc[f], w[f * wst + wi + 1], P.limiter);
-          pred_k(wc, s, 1, c.g, kFast ? rcp_fast(wc[0]) : (T)0, a);
-#pragma unroll
-          for (int f = 0; f < 5; ++f) {
-            const T e = dt2 * a[f] * dxi;                  // muscl.f90:68
-            fm[f] = face_minus(wc[f], s[f], e);
-            fp[f] = face_plus(wc[f], s[f], e);
-          }
-        } else {
-#pragma unroll
-          for (int f = 0; f < 5; ++f) fm[f] = fp[f] = wc[f];
-        }
-        if (cc > i0 - 1) {
-          T fr[NF];
-          riemann_k<T, NF, 1>(fp_prev, fm, fr, P.solver, c, err);   // interface cc-1/2
-          if (cc - 1 >= i0) {
-            T qv[6], wd[5];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) qv[f] = qs[f * n + cc - 1];
-            if (de) {
-              unsigned e2 = 0;
-              prim_k(qv, wd, c, P, de, e2);
-            }
-#pragma unroll
-            for (int f = 0; f < NF; ++f) qs[f * n + cc - 1] = qv[f] + dtdx * (flo[f] - fr[f]);
-          }
-#pragma unroll
-          for (int f = 0; f < NF; ++f) flo[f] = fr[f];
-        }
-#pragma unroll
-        for (int f = 0; f < 5; ++f) fp_prev[f] = fp[f];
-      }
-    }
+    dt = d;
+    t = tt;
+    go = g2;
+    // ---- phase 2: the update
+    tube_sweep<T, NF, NT>(qs, w, n, P, c, de, dt, err);
     ++steps;
-    if (err) atomicOr(s_err, err);
-    __syncthreads();
-    if (!go || *s_err) break;     // a Riemann error stops the tube after its step
+    if (__syncthreads_or(err != 0) || !go) break;   // a Riemann error stops the tube after its step
   }
+  if (err) atomicOr(s_err, err);
   // write back
   for (int f = 0; f < NF; ++f)
     for (int i = tid; i < n; i += NT) A.q[(size_t)f * A.ntot + off + i] = qs[f * n + i];
@@ -211,8 +250,7 @@ template <typename T, int NF, int NT>
 __global__ void __launch_bounds__(NT) k_tubes(BatchArgs<T> A) {
   extern __shared__ __align__(16) unsigned char sraw[];
   __shared__ int s_tube;
-  __shared__ double red[3 * (NT / 32)];
-  __shared__ double bc[4];
+  __shared__ T red[NT / 32];
   __shared__ unsigned s_err;
   for (;;) {
     if (threadIdx.x == 0) {
@@ -239,7 +277,75 @@ __global__ void __launch_bounds__(NT) k_tubes(BatchArgs<T> A) {
       qs = A.gscratch + (size_t)blockIdx.x * (size_t)(NF + 5) * (A.nmax + 4);
       w = qs + (size_t)NF * (A.nmax + 4);
     }
-    tube_run<T, NF, NT>(A, qs, w, tb, red, bc, &s_err);
+    tube_run<T, NF, NT>(A, qs, w, tb, red, &s_err);
+  }
+}
+
+// nsteps steps of a resident 1D grid by one CTA (the loop main.f90:109-155
+// with the control block's scalars): the state in shared memory between them
+// (q_shared), or in place in HBM with its primitives in shared memory.
+// Bound: the latency of a step's dependent chain (primitives, block maximum,
+// dt, faces, solve, update; two barriers), where five launches per step cost
+// 10 us however small the grid.
+template <typename T, int NF, int NT>
+__global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q, GridCtl* ctl, int nsteps,
+                                                int q_shared) {
+  extern __shared__ __align__(16) unsigned char sraw[];
+  __shared__ T red[NT / 32];
+  __shared__ unsigned s_err;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int n = P.nx;
+  T* w = reinterpret_cast<T*>(sraw);
+  T* qs = q_shared ? w + 5 * (n + 4) : q;
+  const Gas<T> c = Gas<T>::make(P);
+  const bool de = NF == 6 && P.dualenergy != 0;
+  const double tend = ctl->tend;
+  double t = ctl->t, dt = ctl->dt;
+  int go = ctl->go, active = ctl->active, k = 0;
+  const int dump = ctl->dump;
+  const unsigned err0 = ctl->err;
+  unsigned err = 0;
+  if (tid == 0) s_err = err0;
+  if (q_shared)
+    for (int i = tid; i < NF * n; i += NT) qs[i] = q[i];
+  __syncthreads();
+  for (int s = 0; s < nsteps; ++s) {
+    // step_begin: nothing more happens once the run has ended or failed
+    active = (go != 0 && s_err == 0 && dump == 0) ? 1 : 0;
+    if (!active) break;
+    const T sm = tube_primitives<T, NF, NT>(qs, w, n, P, c, de, err);
+    if (lane == 0) red[wid] = sm;
+    if (__syncthreads_or(err != 0)) {   // hydrostep's error: no update
+      active = 0;
+      break;
+    }
+    const double smax = (double)warp_max_pos(lane < NT / 32 ? red[lane] : (T)0);
+    unsigned e = 0;
+    double d = cfl_dt1(P, smax, e);
+    if (e) {
+      err |= e;
+      active = 0;
+      break;
+    }
+    update_time(tend, t, d, go);
+    dt = d;
+    tube_sweep<T, NF, NT>(qs, w, n, P, c, de, dt, err);
+    if (__syncthreads_or(err != 0)) break;   // the step is done but not counted
+    ++k;
+  }
+  if (err) atomicOr(&s_err, err);
+  if (q_shared)
+    for (int i = tid; i < NF * n; i += NT) q[i] = qs[i];
+  __syncthreads();
+  if (tid == 0) {
+    ctl->t = t;
+    ctl->dt = dt;
+    ctl->go = go;
+    ctl->active = active;
+    ctl->k += k;
+    ctl->err = s_err;
+    ctl->errnext = 0u;
+    ctl->snext[0] = ctl->snext[1] = ctl->snext[2] = 0ull;
   }
 }
 

@@ -113,6 +113,17 @@ void fused_plan_free(FusedPlan* pl) {
 
 void fused_cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) { pl.cfl(pl, q, ctl, st); }
 
+bool fused_steps1d_fits(const FusedPlan& pl) {
+  if (pl.precision == EVORA_FP32) return f32::steps1d_fits(pl);
+  return pl.strict ? f64s::steps1d_fits(pl) : f64::steps1d_fits(pl);
+}
+
+void fused_steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
+  if (pl.precision == EVORA_FP32) f32::steps1d(pl, q, ctl, nsteps, st);
+  else if (pl.strict) f64s::steps1d(pl, q, ctl, nsteps, st);
+  else f64::steps1d(pl, q, ctl, nsteps, st);
+}
+
 MultiLaunch fused_multi_pick(int precision, int strict, int nf, int* tx, int* ty, int* zc, size_t* smem,
                              int* threads, int* ctas_per_sm) {
   if (precision == EVORA_FP32) return f32::multi_pick(nf, tx, ty, zc, smem, threads, ctas_per_sm);

@@ -342,6 +342,34 @@ void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) {
   else k_cfl_soa<6><<<(int)blocks, 256, 0, st>>>(pl.P, (const TT*)q, pl.n, ctl);
 }
 
+// ---- 1D grids: several steps in one launch
+template <int NF, int NT>
+void steps1d_launch(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, size_t smem, int q_shared,
+                    cudaStream_t st) {
+  cudaFuncSetAttribute(k_steps1d<TT, NF, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_steps1d<TT, NF, NT><<<1, NT, smem, st>>>(pl.P, (TT*)q, ctl, nsteps, q_shared);
+}
+
+// Whether a 1D grid of this size runs k_steps1d (its primitives fit one
+// CTA's shared memory), and its launch.
+constexpr size_t kSteps1dSmem = 224 * 1024;
+bool steps1d_fits(const FusedPlan& pl) {
+  return pl.dim == 1 && 5 * ((size_t)pl.n + 4) * sizeof(TT) <= kSteps1dSmem;
+}
+void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
+  const size_t wb = 5 * ((size_t)pl.n + 4) * sizeof(TT), qb = (size_t)pl.nf * pl.n * sizeof(TT);
+  const int q_shared = wb + qb <= kSteps1dSmem ? 1 : 0;
+  const size_t smem = wb + (q_shared ? qb : 0);
+  // warps for one round of 30 cells each as far as 16 (NT = 512) go
+  if (pl.nf == 5) {
+    if (pl.n <= 240) steps1d_launch<5, 256>(pl, q, ctl, nsteps, smem, q_shared, st);
+    else steps1d_launch<5, 512>(pl, q, ctl, nsteps, smem, q_shared, st);
+  } else {
+    if (pl.n <= 240) steps1d_launch<6, 256>(pl, q, ctl, nsteps, smem, q_shared, st);
+    else steps1d_launch<6, 512>(pl, q, ctl, nsteps, smem, q_shared, st);
+  }
+}
+
 // ---- batched tubes
 template <int NF, int NT>
 void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
@@ -357,6 +385,7 @@ void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
   A.head = pl.head;
   A.budget = pl.budget;
   A.quantum = pl.quantum;
+  A.steps_per_cell = pl.steps_per_cell;
   A.cap = pl.cap;
   A.capw = pl.capw;
   A.gscratch = (TT*)pl.gscratch;
@@ -380,6 +409,7 @@ BatchLaunch batch_pick(int nf, int threads, BatchPlan* pl) {
   if (nf == 5) {
     if (threads == 128) return batch_pick_one<5, 128>(pl);
     if (threads == 512) return batch_pick_one<5, 512>(pl);
+    if (threads == 768) return batch_pick_one<5, 768>(pl);
     return batch_pick_one<5, 256>(pl);
   }
   if (threads == 128) return batch_pick_one<6, 128>(pl);
@@ -399,6 +429,7 @@ int batch_max_ctas_per_sm(int nf, int threads, size_t smem) {
   if (nf == 5) {
     if (threads == 128) return max_ctas_one<5, 128>(smem);
     if (threads == 512) return max_ctas_one<5, 512>(smem);
+    if (threads == 768) return max_ctas_one<5, 768>(smem);
     return max_ctas_one<5, 256>(smem);
   }
   if (threads == 128) return max_ctas_one<6, 128>(smem);

@@ -350,6 +350,27 @@ void flush_step_end(evora_grid* g) {
   g->pending_end = false;
 }
 
+// A 1D grid whose whole step is the hydro update runs its steps inside one
+// kernel (k_steps1d), the step control included; event timing keeps the
+// separate kernels.
+bool steps1d_grid(const evora_grid* g) {
+  return !reference_backend(g) && !g->timing && !g->gravity && !g->floors && !g->conduction &&
+         !g->P.supercomoving && !g->P.cooldt && fused_steps1d_fits(g->plan);
+}
+
+int enqueue_steps1d(evora_grid* g, int nsteps) {
+  flush_step_end(g);
+  while (nsteps > 0) {
+    const int chunk = nsteps < 4096 ? nsteps : 4096;   // a launch stays in the tens of milliseconds
+    fused_steps1d(g->plan, g->qbuf[g->cur], g->ctl, chunk, g->stream);
+    g->launches += 1;
+    nsteps -= chunk;
+  }
+  g->cfl_fresh = false;
+  CU(cudaGetLastError());
+  return 0;
+}
+
 int enqueue_fused_step(evora_grid* g) {
   cudaStream_t st = g->stream;
   const bool use_next = g->cfl_fresh;
@@ -709,6 +730,11 @@ int evora_grid_step(evora_grid* g, int32_t nsteps, int32_t sync) {
   if (g->multigrid) {
     set_error_message("evora_grid_step: the grid is stepped by its multi-grid batch");
     return EVORA_ERR_ARG;
+  }
+  if (nsteps > 0 && steps1d_grid(g)) {
+    int rc = enqueue_steps1d(g, nsteps);
+    if (rc) return rc;
+    nsteps = 0;
   }
   // Several steps on a capturable stream replay graphs of at most 32 steps
   // (instantiating a graph costs with its node count; replays are cheap).
