@@ -28,6 +28,8 @@
 // the slot (same code, generic pointers).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "batch.h"
 #include "fused_kernel.cuh"
 
@@ -281,72 +283,154 @@ __global__ void __launch_bounds__(NT) k_tubes(BatchArgs<T> A) {
   }
 }
 
-// nsteps steps of a resident 1D grid by one CTA (the loop main.f90:109-155
-// with the control block's scalars): the state in shared memory between them
-// (q_shared), or in place in HBM with its primitives in shared memory.
-// Bound: the latency of a step's dependent chain (primitives, block maximum,
-// dt, faces, solve, update; two barriers), where five launches per step cost
-// 10 us however small the grid.
+// ---- resident 1D grids: nsteps steps in one launch by one thread-block
+// cluster (the loop main.f90:109-155 with the control block's scalars).
+//
+// Rank r of the cluster keeps the cells [r m, r m + its cells) in shared
+// memory over the whole launch.  Per step it forms the primitives of its
+// cells, stores the two at either end into its neighbours' halos (or, at the
+// ends of the grid, mirrors them into its own) and its warps' maxima and
+// errors into every rank, all through distributed shared memory; one cluster
+// barrier; dt from all maxima; the sweep; one block barrier.  Halos, maxima
+// and errors are double-buffered by the step's parity: a rank that is one
+// barrier ahead writes the other copy.
+// Bound: the latency of the step's dependent chain; a step of separate kernels
+// cost 10 us however small the grid.  1024 FP64 cells: 9.0 -> 2.2 us per step;
+// by size and number of ranks: steps1d_plan (fused_inst.cuh).
+template <typename T, int NT>
+struct LineMax {
+  T smax[2][16 * (NT / 32)];
+  unsigned err[2][16 * (NT / 32)];
+};
+
 template <typename T, int NF, int NT>
-__global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q, GridCtl* ctl, int nsteps,
-                                                int q_shared) {
+__global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q, GridCtl* ctl, int nsteps, int m) {
+  namespace cg = cooperative_groups;
   extern __shared__ __align__(16) unsigned char sraw[];
-  __shared__ T red[NT / 32];
+  __shared__ LineMax<T, NT> mx;
   __shared__ unsigned s_err;
+  constexpr int NW = NT / 32;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank(), nr = (int)cl.num_blocks();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n = P.nx;
-  T* w = reinterpret_cast<T*>(sraw);
-  T* qs = q_shared ? w + 5 * (n + 4) : q;
+  const int x0 = rank * m;
+  const int mine = n - x0 < m ? n - x0 : m;      // >= 2 (the launch sees to it)
+  const int wlen = 5 * (m + 4);                  // one copy of the primitives
+  T* const w0 = reinterpret_cast<T*>(sraw);
+  T* const qs = w0 + 2 * wlen;                   // field-major, stride mine
+  const int wst = mine + 4;
+  // the neighbours' primitives and row strides
+  const bool periodic = P.boundtype == 2;
+  const int lr = rank > 0 ? rank - 1 : (periodic ? nr - 1 : -1);
+  const int ur = rank < nr - 1 ? rank + 1 : (periodic ? 0 : -1);
+  auto cells_of = [&](int r) { return n - r * m < m ? n - r * m : m; };
+  T* const wl = lr >= 0 ? cl.map_shared_rank(w0, lr) : w0;
+  T* const wu = ur >= 0 ? cl.map_shared_rank(w0, ur) : w0;
+  const int ml = lr >= 0 ? cells_of(lr) : mine, mu = ur >= 0 ? cells_of(ur) : mine;
   const Gas<T> c = Gas<T>::make(P);
   const bool de = NF == 6 && P.dualenergy != 0;
   const double tend = ctl->tend;
   double t = ctl->t, dt = ctl->dt;
   int go = ctl->go, active = ctl->active, k = 0;
-  const int dump = ctl->dump;
-  const unsigned err0 = ctl->err;
-  unsigned err = 0;
-  if (tid == 0) s_err = err0;
-  if (q_shared)
-    for (int i = tid; i < NF * n; i += NT) qs[i] = q[i];
-  __syncthreads();
-  for (int s = 0; s < nsteps; ++s) {
-    // step_begin: nothing more happens once the run has ended or failed
-    active = (go != 0 && s_err == 0 && dump == 0) ? 1 : 0;
-    if (!active) break;
-    const T sm = tube_primitives<T, NF, NT>(qs, w, n, P, c, de, err);
-    if (lane == 0) red[wid] = sm;
-    if (__syncthreads_or(err != 0)) {   // hydrostep's error: no update
-      active = 0;
+  const bool runnable = ctl->err == 0 && ctl->dump == 0;
+  unsigned err = 0, err_step = 0;   // of this thread: recorded; of the last sweep, not yet exchanged
+  if (tid == 0) s_err = 0u;
+  for (int f = 0; f < NF; ++f)
+    for (int i = tid; i < mine; i += NT) qs[f * mine + i] = q[(int64_t)f * n + x0 + i];
+  cl.sync();   // every rank has started before any stores into its shared memory
+  for (int s = 0;; ++s) {
+    const int par = s & 1;
+    T* const w = w0 + par * wlen;
+    // another step, unless the run has ended (step_begin); the round after
+    // the last step only exchanges its errors
+    const bool step = s < nsteps && go != 0 && runnable;
+    active = step ? 1 : (s < nsteps ? 0 : active);
+    T smax = (T)0;
+    unsigned e = 0;
+    if (step) {
+      for (int i = tid; i < mine; i += NT) {
+        T qv[6], wv[5];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) qv[f] = qs[f * mine + i];
+        prim_k(qv, wv, c, P, de, e);
+#pragma unroll
+        for (int f = 0; f < 5; ++f) w[f * wst + i + 2] = wv[f];
+        T a;
+        if constexpr (kFast && sizeof(T) == 8) a = sqrt_fast(c.g * wv[4] * rcp_fast(wv[0]));
+        else a = dsqrt(c.g * wv[4] / wv[0]);
+        const T sp = fmax2(fmax2((T)fabs(wv[1]), (T)fabs(wv[2])), (T)fabs(wv[3])) + a;
+        if (sp > smax) smax = sp;
+        // bound (boundary.f90:33-66) and the ranks' halos
+        if (i < 2) {
+          T* d = lr >= 0 ? wl + par * wlen + ml + 2 + i : w + 1 - i;
+          const int st = lr >= 0 ? ml + 4 : wst;
+#pragma unroll
+          for (int f = 0; f < 5; ++f) d[f * st] = wv[f];
+        }
+        if (i >= mine - 2) {
+          const int j = mine - 1 - i;
+          T* d = ur >= 0 ? wu + par * wlen + 1 - j : w + mine + 2 + j;
+          const int st = ur >= 0 ? mu + 4 : wst;
+          const bool flip = ur < 0 && P.boundtype == 3;
+#pragma unroll
+          for (int f = 0; f < 5; ++f) d[f * st] = flip && f >= 1 && f <= 3 ? -wv[f] : wv[f];
+        }
+      }
+      smax = warp_max_pos(smax);
+    }
+    // a sweep's errors in the upper, the primitives' in the lower half
+    const unsigned eall = __reduce_or_sync(0xffffffffu, (err_step << 16) | e);
+    if (lane < nr) {
+      LineMax<T, NT>* r = cl.map_shared_rank(&mx, lane);
+      r->smax[par][rank * NW + wid] = smax;
+      r->err[par][rank * NW + wid] = eall;
+    }
+    cl.sync();
+    T g = (T)0;
+    unsigned ge = 0;
+    for (int i = lane; i < nr * NW; i += 32) {
+      g = fmax2(g, mx.smax[par][i]);
+      ge |= mx.err[par][i];
+    }
+    ge = __reduce_or_sync(0xffffffffu, ge);
+    if (ge >> 16) {   // the last sweep failed: done but not counted, and nothing after it
+      err |= ge >> 16;
+      if (s < nsteps) active = 0;
       break;
     }
-    const double smax = (double)warp_max_pos(lane < NT / 32 ? red[lane] : (T)0);
-    unsigned e = 0;
-    double d = cfl_dt1(P, smax, e);
-    if (e) {
-      err |= e;
+    if (s > 0) ++k;
+    if (!step) break;
+    const double gm = (double)warp_max_pos(g);
+    unsigned ed = ge & 0xffffu;
+    double d = 0.0;
+    if (!ed) d = cfl_dt1(P, gm, ed);
+    if (ed) {         // hydrostep's errors: no update
+      err |= ed;
       active = 0;
       break;
     }
     update_time(tend, t, d, go);
     dt = d;
-    tube_sweep<T, NF, NT>(qs, w, n, P, c, de, dt, err);
-    if (__syncthreads_or(err != 0)) break;   // the step is done but not counted
-    ++k;
+    err_step = 0;
+    tube_sweep<T, NF, NT>(qs, w, mine, P, c, de, dt, err_step);
+    __syncthreads();
   }
-  if (err) atomicOr(&s_err, err);
-  if (q_shared)
-    for (int i = tid; i < NF * n; i += NT) q[i] = qs[i];
+  if (err && lane == 0) atomicOr(&s_err, err);
+  for (int f = 0; f < NF; ++f)
+    for (int i = tid; i < mine; i += NT) q[(int64_t)f * n + x0 + i] = qs[f * mine + i];
   __syncthreads();
-  if (tid == 0) {
+  if (rank == 0 && tid == 0) {
     ctl->t = t;
     ctl->dt = dt;
     ctl->go = go;
     ctl->active = active;
     ctl->k += k;
-    ctl->err = s_err;
+    ctl->err |= s_err;
     ctl->errnext = 0u;
     ctl->snext[0] = ctl->snext[1] = ctl->snext[2] = 0ull;
   }
+  cl.sync();   // no rank leaves while its shared memory may be written
 }
 
 }  // namespace EVORA_FNS

@@ -18,11 +18,12 @@ struct Inst {
   int (*tiles)();
   void (*cfl)(const FusedPlan&, const void*, GridCtl*, cudaStream_t);
   bool (*fits)(const HydroParams&, int, int, int);
+  int (*steps1d_plan)(const FusedPlan&);
 };
 Inst inst_of(int precision, int strict) {
-  if (precision == EVORA_FP32) return {f32::pick, f32::tiles, f32::cfl, f32::tile_fits};
-  if (strict) return {f64s::pick, f64s::tiles, f64s::cfl, f64s::tile_fits};
-  return {f64::pick, f64::tiles, f64::cfl, f64::tile_fits};
+  if (precision == EVORA_FP32) return {f32::pick, f32::tiles, f32::cfl, f32::tile_fits, f32::steps1d_plan};
+  if (strict) return {f64s::pick, f64s::tiles, f64s::cfl, f64s::tile_fits, f64s::steps1d_plan};
+  return {f64::pick, f64::tiles, f64::cfl, f64::tile_fits, f64::steps1d_plan};
 }
 }  // namespace
 
@@ -90,6 +91,7 @@ int fused_plan(const HydroParams& P, int precision, int nf, int strict, FusedPla
   int tile = 0;
   if (const char* e = getenv("EVORA_TILE")) tile = atoi(e);
   fused_set_tile(pl, tile);
+  pl->ranks1d = inst_of(precision, strict).steps1d_plan(*pl);
   int64_t nb = (pl->n + 255) / 256;
   pl->nblk_tot = (int)(nb > 148 * 4 ? 148 * 4 : nb);
   pl->alloc_stream = astream;
@@ -112,11 +114,6 @@ void fused_plan_free(FusedPlan* pl) {
 }
 
 void fused_cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) { pl.cfl(pl, q, ctl, st); }
-
-bool fused_steps1d_fits(const FusedPlan& pl) {
-  if (pl.precision == EVORA_FP32) return f32::steps1d_fits(pl);
-  return pl.strict ? f64s::steps1d_fits(pl) : f64::steps1d_fits(pl);
-}
 
 void fused_steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
   if (pl.precision == EVORA_FP32) f32::steps1d(pl, q, ctl, nsteps, st);

@@ -35,6 +35,7 @@ struct FusedPlan {
   // writes into ctl->snext (2D and 3D kernels), so that step needs no CFL
   // kernel
   int cfl_fused = 0;
+  int ranks1d = 0;   // 1D: CTAs of the cluster that runs several steps in one launch (0: the grid does not fit one)
 };
 
 // Chooses tiles and the kernel instantiation; allocates small scratch.
@@ -52,9 +53,8 @@ void fused_cfl(const FusedPlan& plan, const void* q, GridCtl* ctl, cudaStream_t 
 // The fused MUSCL-Hancock update (primitive, bound, compevo, sweep).
 void fused_update(const FusedPlan& plan, const void* qin, void* qout, GridCtl* ctl, cudaStream_t st);
 
-// 1D grids without physics after the update: whether `nsteps` steps of the
-// state q (in place) run in one launch, and that launch.
-bool fused_steps1d_fits(const FusedPlan& plan);
+// 1D grids without physics after the update, plan.ranks1d > 0: `nsteps`
+// steps of the state q, in place, in one launch.
 void fused_steps1d(const FusedPlan& plan, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);
 
 // Layout conversions between the reference q(6, nx, ny, nz) (FP64) and the
@@ -124,7 +124,7 @@ MultiLaunch fused_multi_pick(int precision, int strict, int nf, int* tx, int* ty
   bool tile_fits(const HydroParams& P, int nf, int dim, int tile);                           \
   MultiLaunch multi_pick(int nf, int* tx, int* ty, int* zc, size_t* smem, int* threads, int* ctas_per_sm); \
   void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st);                \
-  bool steps1d_fits(const FusedPlan& pl);                                                    \
+  int steps1d_plan(const FusedPlan& pl);                                                     \
   void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);      \
   }
 EVORA_DECLARE_FUSED_NS(f64)

@@ -343,30 +343,81 @@ void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) {
 }
 
 // ---- 1D grids: several steps in one launch
+constexpr size_t kSteps1dSmem = 220 * 1024;
+size_t steps1d_smem(int nf, int m) { return ((size_t)10 * (m + 4) + (size_t)nf * m) * sizeof(TT); }
+
 template <int NF, int NT>
-void steps1d_launch(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, size_t smem, int q_shared,
-                    cudaStream_t st) {
+void steps1d_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int ranks, size_t smem, cudaStream_t st) {
   cudaFuncSetAttribute(k_steps1d<TT, NF, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_steps1d<TT, NF, NT><<<1, NT, smem, st>>>(pl.P, (TT*)q, ctl, nsteps, q_shared);
+  if (ranks > 8) cudaFuncSetAttribute(k_steps1d<TT, NF, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(ranks);
+  cfg->blockDim = dim3(NT);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = st;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = ranks;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
 }
 
-// Whether a 1D grid of this size runs k_steps1d (its primitives fit one
-// CTA's shared memory), and its launch.
-constexpr size_t kSteps1dSmem = 224 * 1024;
-bool steps1d_fits(const FusedPlan& pl) {
-  return pl.dim == 1 && 5 * ((size_t)pl.n + 4) * sizeof(TT) <= kSteps1dSmem;
+template <int NF, int NT>
+void steps1d_launch(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, int m, cudaStream_t st) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  steps1d_config<NF, NT>(&cfg, &at, pl.ranks1d, steps1d_smem(NF, m), st);
+  cudaLaunchKernelEx(&cfg, k_steps1d<TT, NF, NT>, pl.P, (TT*)q, ctl, nsteps, m);   // errors: cudaGetLastError
 }
+
+template <int NF>
+bool steps1d_wide(int m) {   // whether this device schedules clusters of 16 such CTAs
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  steps1d_config<NF, 512>(&cfg, &at, 16, steps1d_smem(NF, m), nullptr);
+  int count = 0;
+  const bool ok = cudaOccupancyMaxActiveClusters(&count, k_steps1d<TT, NF, 512>, &cfg) == cudaSuccess;
+  cudaGetLastError();
+  return ok && count > 0;
+}
+
+// Ranks of the cluster that k_steps1d runs a 1D grid with, 0 if the grid
+// does not fit one.  us per step, FP64 / FP32, by ranks:
+//      cells        1            2            4            8           16
+//         64  1.73 / 1.34  1.78 / 1.42  1.85 / 1.46  1.97 / 1.57  2.25 / 1.85
+//        200  2.01 / 1.49  1.80 / 1.42  1.84 / 1.44  1.96 / 1.59  2.24 / 1.82
+//        400  2.78 / 1.84  2.07 / 1.55  1.82 / 1.46  1.99 / 1.59  2.26 / 1.84
+//       1024  5.24 / 2.93  3.49 / 2.18  2.39 / 1.76  2.18 / 1.64  2.23 / 1.74
+//       8000   - / -        - / -        - / 4.63    5.51 / 3.21  4.55 / 3.43
+//      23000   - / -        - / -        - / -        - / 6.00    7.25 / 4.59
+// against 9 to 13 with separate kernels.  The smallest count within 5 % of
+// the best up to 8, the largest portable cluster; 16, where the device has
+// room for it, once a rank of 8 would hold more than 1000 (FP64) or 2000
+// (FP32) cells.
+int steps1d_plan(const FusedPlan& pl) {
+  if (pl.dim != 1) return 0;
+  auto per_rank = [&](int r) { return (int)((pl.n + r - 1) / r); };
+  auto fits = [&](int r) {
+    const int m = per_rank(r);
+    return pl.n - (int64_t)(r - 1) * m >= 2 && steps1d_smem(pl.nf, m) <= kSteps1dSmem;
+  };
+  int r = pl.n <= 96 ? 1 : (pl.n <= 300 ? 2 : (pl.n <= 700 ? 4 : 8));
+  if (per_rank(8) > (sizeof(TT) == 8 ? 1000 : 2000) && fits(16) &&
+      (pl.nf == 5 ? steps1d_wide<5>(per_rank(16)) : steps1d_wide<6>(per_rank(16))))
+    return 16;
+  return fits(r) ? r : 0;
+}
+
 void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
-  const size_t wb = 5 * ((size_t)pl.n + 4) * sizeof(TT), qb = (size_t)pl.nf * pl.n * sizeof(TT);
-  const int q_shared = wb + qb <= kSteps1dSmem ? 1 : 0;
-  const size_t smem = wb + (q_shared ? qb : 0);
-  // warps for one round of 30 cells each as far as 16 (NT = 512) go
+  // warps for one round of 30 cells each, as far as 16 of them go
+  const int m = (int)((pl.n + pl.ranks1d - 1) / pl.ranks1d);
   if (pl.nf == 5) {
-    if (pl.n <= 240) steps1d_launch<5, 256>(pl, q, ctl, nsteps, smem, q_shared, st);
-    else steps1d_launch<5, 512>(pl, q, ctl, nsteps, smem, q_shared, st);
+    if (m <= 240) steps1d_launch<5, 256>(pl, q, ctl, nsteps, m, st);
+    else steps1d_launch<5, 512>(pl, q, ctl, nsteps, m, st);
   } else {
-    if (pl.n <= 240) steps1d_launch<6, 256>(pl, q, ctl, nsteps, smem, q_shared, st);
-    else steps1d_launch<6, 512>(pl, q, ctl, nsteps, smem, q_shared, st);
+    if (m <= 240) steps1d_launch<6, 256>(pl, q, ctl, nsteps, m, st);
+    else steps1d_launch<6, 512>(pl, q, ctl, nsteps, m, st);
   }
 }
 

@@ -351,11 +351,11 @@ void flush_step_end(evora_grid* g) {
 }
 
 // A 1D grid whose whole step is the hydro update runs its steps inside one
-// kernel (k_steps1d), the step control included; event timing keeps the
+// launch (k_steps1d), the step control included; event timing keeps the
 // separate kernels.
 bool steps1d_grid(const evora_grid* g) {
   return !reference_backend(g) && !g->timing && !g->gravity && !g->floors && !g->conduction &&
-         !g->P.supercomoving && !g->P.cooldt && fused_steps1d_fits(g->plan);
+         !g->P.supercomoving && !g->P.cooldt && g->plan.ranks1d > 0;
 }
 
 int enqueue_steps1d(evora_grid* g, int nsteps) {

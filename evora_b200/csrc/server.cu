@@ -596,13 +596,15 @@ int evora_server_create(const evora_params* base, int32_t precision, int32_t fla
     pl.nmax = max_tube_cells;
     pl.cell_updates = s->cu;
     const size_t per_cell = (size_t)(s->nf + 5) * s->esize();
-    // one CTA of 512 threads per SM, the largest shared-memory staging
+    // one CTA of 768 threads per SM (512 with 6 fields), the largest
+    // shared-memory staging
+    const int nt = s->nf == 5 ? 768 : 512;
     pl.cap = std::min(max_tube_cells, (int)((227 * 1024 - 4096) / per_cell) - 4);
-    s->launch = batch_pick_for(precision, (flags & EVORA_STRICT) != 0, s->nf, 512, &pl);
+    s->launch = batch_pick_for(precision, (flags & EVORA_STRICT) != 0, s->nf, nt, &pl);
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int per_sm = batch_ctas_per_sm(precision, (flags & EVORA_STRICT) != 0, s->nf, 512, pl.smem);
+    int per_sm = batch_ctas_per_sm(precision, (flags & EVORA_STRICT) != 0, s->nf, nt, pl.smem);
     pl.ctas = std::max(1, sms * std::max(1, per_sm));
     if (max_tube_cells > pl.cap) {
       size_t need = (size_t)pl.ctas * (size_t)(s->nf + 5) * (size_t)(max_tube_cells + 4) * s->esize();
