@@ -46,20 +46,6 @@ __device__ __forceinline__ double cfl_dt1(const HydroParams& P, double smax, uns
   return dt;
 }
 
-// The largest of a non-negative value (no NaN) over a warp, or over red[0..NW)
-// for every lane: values >= 0 order like their bits, which one (FP32) or two
-// (FP64: high words, then the low words of those that have the largest)
-// warp reductions of unsigned words take.
-__device__ __forceinline__ float warp_max_pos(float v) {
-  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
-}
-__device__ __forceinline__ double warp_max_pos(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  return __hiloint2double((int)mh, (int)ml);
-}
-
 // Primitives of the n cells of a tube and its 2 + 2 ghosts (the index map of
 // bound) into w (field-major, stride n + 4); returns this thread's maximum of
 // |u_d| + a over the cells (timestep.f90:40-43), reduced over its warp.  One

@@ -11,6 +11,7 @@
 #include "conduction.h"
 #include "fused.h"
 #include "fused_kernel.cuh"
+#include "fused_march.cuh"
 #include "fused_tma.cuh"
 #if EVORA_PRECISION_F32
 #include "fused_pair.cuh"
@@ -28,8 +29,8 @@ using TT = EVORA_T;
 // measured no faster than the three-barrier march, 3.24 against 3.23 ms per
 // 256^3 launch).  Entry 0 is the
 // default for grids the TMA kernel does not take; evora_grid_autotune times
-// all entries on the grid itself.  The 3D kernels are instantiated for every
-// entry, the 1D and 2D ones for entry 0 only.
+// all entries on the grid itself.  The entries are the 3D kernels'; 1D and 2D
+// grids have one kernel each.
 template <int I> struct Tile;
 #if EVORA_PRECISION_F32
 template <> struct Tile<0> { static constexpr int TX = 32, TY = 8, ZC = 32, MINB = 3, TMA = 0, PIPE = 1; };
@@ -94,11 +95,36 @@ bool tma_fits(const HydroParams& P, int dim) {
   return dim == 3 && P.nx % TX == 0 && P.ny % TY == 0 && ((size_t)P.nx * sizeof(TT)) % 16 == 0;
 }
 
+// Launches a 2D update.  With a step control tail the launch may overlap the
+// end of the previous one (step_head), which hides the gap between two
+// launches (1024^2 FP64: 78 -> 72 us).  In 3D the same lost: CTAs placed while
+// the previous update's last ones still run crowd onto the SMs that are free
+// first (100 x 75 x 61 FP32: 90 -> 112 us).
+template <class Kernel, class... Args>
+void launch_step(const FusedPlan& pl, Kernel k, int threads, size_t smem, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = pl.grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = pl.tail ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, args...);   // errors: cudaGetLastError
+}
+
 template <int NF, int DIM, int I>
 void launch(const FusedPlan& pl, const void* qin, void* qout, GridCtl* ctl, cudaStream_t st) {
-  FusedArgs<TT> A{pl.P, (const TT*)qin, (TT*)qout, ctl, pl.n, pl.cfl_fused, pl.zc};
+  FusedArgs<TT> A{pl.P, (const TT*)qin, (TT*)qout, ctl, pl.n, pl.cfl_fused, pl.zc, pl.tail};
   if constexpr (DIM == 1) {
     k_fused1d<TT, NF><<<pl.grid, pl.threads, 0, st>>>(A);
+  } else if constexpr (DIM == 2) {
+    if (pl.P.limiter == 1 && pl.P.solver == 2 && pl.P.secondorder)
+      launch_step(pl, k_march2d<TT, NF, true>, pl.threads, 0, st, A);
+    else
+      launch_step(pl, k_march2d<TT, NF, false>, pl.threads, 0, st, A);
   } else {
     using C = Tile<I>;
 #if EVORA_PRECISION_F32
@@ -133,6 +159,9 @@ template <int NF, int DIM, int I>
 FusedLaunch pick_one(int* tx, int* ty, int* zc, size_t* smem, int* threads, int* minb) {
   if constexpr (DIM == 1) {
     *tx = 128; *ty = 1; *zc = 1; *smem = 0; *threads = 128; *minb = 1;
+  } else if constexpr (DIM == 2) {
+    // the march: warps of kMarchCols columns, zc rows each (set by the plan)
+    *tx = kMarchCols; *ty = 1; *zc = 1; *smem = 0; *threads = 32 * kMarchWarps; *minb = 1;
   } else {
     using C = Tile<I>;
     *tx = C::TX; *ty = C::TY; *zc = DIM == 3 ? C::ZC : 1; *minb = C::MINB;

@@ -64,7 +64,8 @@ struct FusedArgs {
   GridCtl* ctl;     // dt, active flag, error mask
   int64_t n;        // cells per field
   int cfl_next = 0; // 1: reduce the next step's CFL maxima into ctl->snext
-  int zc = 0;       // planes per CTA (0: the instantiation's ZC)
+  int zc = 0;       // planes per CTA (0: the instantiation's ZC); 2D march: rows per warp
+  int tail = 0;     // what the last CTA does for the step control (step_tail)
 };
 
 // Boundary index map of one axis (0-based), boundary.f90:26-113: g in
@@ -270,17 +271,19 @@ __device__ __forceinline__ void cfl_speeds(const T* qs, const HydroParams& P, bo
 // Slopes, predictor and face states of one cell.  get(f, dx, dy, dz) reads
 // primitive f of the neighbour at offset (dx, dy, dz) (one axis at a time).
 // DIM = 2 or 3 selects the 2D (muscl.f90:70-88) or 3D (89-111) predictor.
-template <typename T, int DIM, typename Get>
+// OPT: the usual options (minmod, second order) as constants.
+template <typename T, int DIM, bool OPT = false, typename Get>
 __device__ __forceinline__ void cell_faces_g(Get get, const HydroParams& P, T dt2, T* wv, T (*face)[2][5]) {
+  const int limiter = OPT ? 1 : P.limiter;
   T sx[5], sy[5], sz[5];
 #pragma unroll
   for (int f = 0; f < 5; ++f) {
     wv[f] = get(f, 0, 0, 0);
-    sx[f] = slope_k(get(f, -1, 0, 0), wv[f], get(f, 1, 0, 0), P.limiter);
-    sy[f] = slope_k(get(f, 0, -1, 0), wv[f], get(f, 0, 1, 0), P.limiter);
-    if (DIM == 3) sz[f] = slope_k(get(f, 0, 0, -1), wv[f], get(f, 0, 0, 1), P.limiter);
+    sx[f] = slope_k(get(f, -1, 0, 0), wv[f], get(f, 1, 0, 0), limiter);
+    sy[f] = slope_k(get(f, 0, -1, 0), wv[f], get(f, 0, 1, 0), limiter);
+    if (DIM == 3) sz[f] = slope_k(get(f, 0, 0, -1), wv[f], get(f, 0, 0, 1), limiter);
   }
-  if (!P.secondorder) {
+  if (!OPT && !P.secondorder) {
     // first-order Godunov: the face states are the cell averages (sweep,
     // muscl.f90:198-201, 207-210)
 #pragma unroll
@@ -892,6 +895,92 @@ __device__ __forceinline__ void fused_cell1d(const FusedArgs<T>& A, int i) {
 }
 
 #if !defined(EVORA_HOST_EMU)
+// The largest of a non-negative value (no NaN) over a warp, or over red[0..NW)
+// for every lane: values >= 0 order like their bits, which one (FP32) or two
+// (FP64: high words, then the low words of those that have the largest)
+// warp reductions of unsigned words take.
+__device__ __forceinline__ float warp_max_pos(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warp_max_pos(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+// The step control after a hydro-only 2D update (no physics, not comoving), by
+// the last CTA to finish: A.tail = 1 the step's end, and the next step's
+// begin and time from the maxima this update reduced (k_step_control's work,
+// grid.cu, in its order); A.tail = 2 the end alone; 0 nothing.  Saves the
+// control kernel's launch between two updates (64^2 FP32: 8.8 -> 7.1 us per
+// step, with the march).  The 3D updates keep the control kernel: theirs take
+// 80 us and more, and the tail gained 0.5 % in FP64 and lost 1 to 2 % in FP32.
+__device__ __forceinline__ void hydro_control(const HydroParams& P, GridCtl* ctl, int tail, long long k, int active,
+                                              int go, int dump, double t, double tend) {
+  // what the update's CTAs wrote, past this SM's L1
+  unsigned err = __ldcg(&ctl->err);
+  const unsigned errnext = __ldcg(&ctl->errnext);
+  unsigned long long s[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) s[i] = __ldcg(&ctl->snext[i]);
+  if (active && err == 0) ctl->k = k + 1;
+  if (tail != 1) return;
+  err |= errnext;
+  active = (go != 0 && err == 0 && dump == 0) ? 1 : 0;
+  if (active) {
+    unsigned e = 0;
+    double dt = cfl_dt(P, __longlong_as_double((long long)s[0]), __longlong_as_double((long long)s[1]),
+                       __longlong_as_double((long long)s[2]), 1e99, e);
+    if (e) {
+      err |= e;
+      active = 0;
+    } else {
+      update_time(tend, t, dt, go);
+      ctl->t = t;
+      ctl->dt = dt;
+      ctl->go = go;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    ctl->smax[i] = s[i];
+    ctl->snext[i] = 0ull;
+  }
+  ctl->errnext = 0u;
+  ctl->err = err;
+  ctl->active = active;
+}
+
+// Start of an update that may be launched while the previous one still runs
+// (programmatic dependent launch): lets the next one start being launched and
+// waits until the previous one is complete.  Without that launch attribute
+// both are no-ops.
+__device__ __forceinline__ void step_head() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+// Called by all threads of every CTA once the tile is done.
+template <typename T>
+__device__ __forceinline__ void step_tail(const FusedArgs<T>& A) {
+  if (!A.tail) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    GridCtl* ctl = A.ctl;
+    // fields that only the step control writes, read while the fence waits
+    const long long k = ctl->k;
+    const int active = ctl->active, go = ctl->go, dump = ctl->dump;
+    const double t = ctl->t, tend = ctl->tend;
+    __threadfence();   // this CTA's maxima and errors before its ticket
+    if (atomicAdd(&ctl->ticket, 1u) == gridDim.x * gridDim.y * gridDim.z - 1) {
+      __threadfence();
+      ctl->ticket = 0u;
+      hydro_control(A.P, ctl, A.tail, k, active, go, dump, t, tend);
+    }
+  }
+}
+
 template <typename T, int NF>
 __global__ void __launch_bounds__(128) k_fused1d(FusedArgs<T> A) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.P.nx; i += gridDim.x * blockDim.x)

@@ -64,8 +64,12 @@ struct evora_grid {
   std::map<long long, cudaGraphExec_t> graphs;
   std::map<long long, int64_t> graph_launches;   // kernel launches per replay, by key
   // the last enqueued step's closing control (step_end) is deferred into the
-  // next step's first control kernel or a flush
+  // next step's first control kernel or a flush (steps with physics after the
+  // update, and timed ones)
   bool pending_end = false;
+  // the last enqueued update also does the next step's begin and time
+  // (step_tail); only between the steps of one evora_grid_step call or graph
+  bool control_done = false;
   // the previous update reduced the CFL maxima of the current state into
   // ctl->snext; any other change of the state clears this
   bool cfl_fresh = false;
@@ -371,10 +375,23 @@ int enqueue_steps1d(evora_grid* g, int nsteps) {
   return 0;
 }
 
-int enqueue_fused_step(evora_grid* g) {
+// A 2D step that is the hydro update alone: its update reduces the next
+// step's CFL maxima and runs the step control in its last CTA (step_tail).
+bool hydro_only_2d(const evora_grid* g) {
+  return g->plan.dim == 2 && g->plan.cfl_fused && !g->P.supercomoving && !g->P.cooldt && !g->P.conduction;
+}
+
+// more: another step follows at once (in this call or graph).
+int enqueue_fused_step(evora_grid* g, bool more) {
   cudaStream_t st = g->stream;
   const bool use_next = g->cfl_fresh;
-  if (use_next && !g->P.cooldt) {
+  g->plan.tail = hydro_only_2d(g) && !g->timing ? (more ? 1 : 2) : 0;
+  if (g->control_done) {
+    g->control_done = false;
+    g->launches += 1;   // the update
+    mark(g);
+    mark(g);
+  } else if (use_next && !g->P.cooldt) {
     // the previous step's end, this step's begin and time in one launch
     k_step_control<<<1, 1, 0, st>>>(g->P, g->ctl, g->pending_end ? 1 : 0);
     g->pending_end = false;
@@ -434,7 +451,10 @@ int enqueue_fused_step(evora_grid* g) {
     g->launches += 1;
   }
   mark(g);
-  g->pending_end = true;   // k_step_end, deferred (flush_step_end, k_step_control)
+  // k_step_end, deferred (flush_step_end, k_step_control) unless the update did it
+  g->pending_end = g->plan.tail == 0;
+  g->control_done = g->plan.tail == 1;
+  g->plan.tail = 0;
   CU(cudaGetLastError());
   // The swap is unconditional on the host; an inactive step copies q through
   // unchanged (fused_update does that when the step is inactive).
@@ -745,7 +765,7 @@ int evora_grid_step(evora_grid* g, int32_t nsteps, int32_t sync) {
     nsteps -= chunk;
   }
   for (int i = 0; i < nsteps; ++i) {
-    int rc = reference_backend(g) ? enqueue_reference_step(g) : enqueue_fused_step(g);
+    int rc = reference_backend(g) ? enqueue_reference_step(g) : enqueue_fused_step(g, i + 1 < nsteps);
     if (rc) return rc;
   }
   flush_step_end(g);
@@ -773,10 +793,11 @@ int graph_steps(evora_grid* g, int nsteps) {
       int rc = 0;
       const int64_t launches0 = g->launches;
       for (int i = 0; i < nsteps && !rc; ++i)
-        rc = reference_backend(g) ? enqueue_reference_step(g) : enqueue_fused_step(g);
+        rc = reference_backend(g) ? enqueue_reference_step(g) : enqueue_fused_step(g, i + 1 < nsteps);
       if (!rc) flush_step_end(g);
       cudaError_t e = cudaStreamEndCapture(g->stream, &graph);
       g->pending_end = false;
+      g->control_done = false;
       g->cur = start;
       g->cfl_fresh = fresh;
       const int64_t per_replay = g->launches - launches0;

@@ -61,6 +61,7 @@ struct GridCtl {
   int k4;        // the next dump_redshift index updatetime tests (main.f90:33)
   double dump_redshift[EVORA_NDUMP];
   ChemCoef coef;   // the chemistry's rate coefficients of the current step
+  unsigned ticket; // CTAs of the running update that are done (step_tail)
 };
 
 __device__ __forceinline__ bool ctl_skip(const GridCtl* ctl) {
@@ -587,7 +588,12 @@ __host__ __device__ inline double cfl_dt(const HydroParams& P, double sx, double
   double v = 1e6;
   double vx = P.dx / sx, vy = P.dy / sy, vz = P.dz / sz;
   v = fmin2(fmin2(fmin2(vx, vy), vz), v);
-  double dt = fmin2(P.cfl * v, dt_in);
+#if defined(__CUDA_ARCH__)
+  const double cv = __dmul_rn(P.cfl, v);   // never contracted with the sum t + dt
+#else
+  const double cv = P.cfl * v;
+#endif
+  double dt = fmin2(cv, dt_in);
   if (dt <= 0.0) err |= EVORA_ERR_DT;
   return dt;
 }
