@@ -104,14 +104,14 @@ __device__ __forceinline__ void tube_sweep_opt(T* qs, const T* w, int n, const H
     for (int f = 0; f < 5; ++f) wc[f] = w[f * wst + wi];
     if (secondorder) {
       T s[5], a[5];
+      with_limiter<false>(limiter, [&](auto lim) {
 #pragma unroll
-      for (int f = 0; f < 5; ++f) s[f] = slope_k(w[f * wst + wi - 1], wc[f], w[f * wst + wi + 1], limiter);
+        for (int f = 0; f < 5; ++f) s[f] = slope_k(w[f * wst + wi - 1], wc[f], w[f * wst + wi + 1], lim);
+      });
       pred_k(wc, s, 1, c.g, kFast ? rcp_fast(wc[0]) : (T)0, a);
 #pragma unroll
       for (int f = 0; f < 5; ++f) {
-        const T e = dt2 * a[f] * dxi;                  // muscl.f90:68
-        fm[f] = face_minus(wc[f], s[f], e);
-        fp[f] = face_plus(wc[f], s[f], e);
+        faces1d(wc[f], s[f], dt2, a[f], dxi, fm[f], fp[f]);
       }
     } else {
 #pragma unroll
@@ -135,7 +135,7 @@ __device__ __forceinline__ void tube_sweep_opt(T* qs, const T* w, int n, const H
         prim_k(qv, wd, c, P, de, e2);   // dual-energy resync of q (comp.f90:60-72)
       }
 #pragma unroll
-      for (int f = 0; f < NF; ++f) qs[f * n + cc] = qv[f] + dtdx * (flo[f] - fhi[f]);
+      for (int f = 0; f < NF; ++f) qs[f * n + cc] = axpy_k<kFast>(qv[f], dtdx, flo[f] - fhi[f]);
     }
   }
 }

@@ -23,11 +23,11 @@ namespace EVORA_FNS {
 using TT = EVORA_T;
 
 // Tile table of this precision: (TX, TY, ZC, CTAs per SM, TMA, PIPE).
-// TMA = 1: the tensor-staged 3D kernel of fused_tma.cuh, for grids tiled by
-// whole tiles (the plan falls back to entry 0 elsewhere).  PIPE = 1: the
-// two-barrier pipelined 3D march of fused_kernel.cuh (FP32; in FP64 it
-// measured no faster than the three-barrier march, 3.24 against 3.23 ms per
-// 256^3 launch).  Entry 0 is the
+// TMA = 1: the tensor-staged 3D kernel of fused_tma.cuh (FP32; in FP64 it took
+// 3.35 ms per 256^3 launch against 2.11), for grids tiled by whole tiles (the
+// plan falls back to entry 0 elsewhere).  PIPE = 1: the two-barrier pipelined
+// 3D march of fused_kernel.cuh (FP32; in FP64 it measured no faster than the
+// three-barrier march, 2.113 against 2.114 ms per 256^3 launch).  Entry 0 is the
 // default for grids the TMA kernel does not take; evora_grid_autotune times
 // all entries on the grid itself.  The entries are the 3D kernels'; 1D and 2D
 // grids have one kernel each.
@@ -46,7 +46,7 @@ template <> struct Tile<0> { static constexpr int TX = 16, TY = 8, ZC = 32, MINB
 template <> struct Tile<1> { static constexpr int TX = 32, TY = 4, ZC = 32, MINB = 3, TMA = 0, PIPE = 0; };
 template <> struct Tile<2> { static constexpr int TX = 16, TY = 8, ZC = 16, MINB = 3, TMA = 0, PIPE = 0; };
 template <> struct Tile<3> { static constexpr int TX = 16, TY = 8, ZC = 64, MINB = 3, TMA = 0, PIPE = 0; };
-template <> struct Tile<4> { static constexpr int TX = 16, TY = 8, ZC = 32, MINB = 2, TMA = 1, PIPE = 0; };
+template <> struct Tile<4> { static constexpr int TX = 16, TY = 8, ZC = 32, MINB = 2, TMA = 0, PIPE = 0; };
 constexpr int kTiles = 5;
 #endif
 
@@ -202,8 +202,8 @@ bool tile_fits(const HydroParams& P, int nf, int dim, int tile) {
     return encode_state_map<5, C5::TX, C5::TY>(P, reinterpret_cast<const void*>((uintptr_t)1 << 20), &map);
   }
 #endif
-  if (tile != 4) return true;
   using C = Tile<4>;
+  if (tile != 4 || C::TMA == 0) return true;
   if (!tma_fits<C::TX, C::TY>(P, dim)) return false;
   // encode against an aligned dummy address: only shapes and strides are checked
   CUtensorMap map;

@@ -33,6 +33,8 @@
 // logic can be checked against the CPU oracle without a GPU.
 #pragma once
 
+#include <type_traits>
+
 #include "hydro_math.cuh"
 
 #ifdef EVORA_HOST_EMU
@@ -164,6 +166,15 @@ __device__ __forceinline__ T slope_k(T wl, T w, T wr, int limiter) {
   else return slope1(wl, w, wr, limiter);
 }
 
+// Calls f with the limiter as a compile-time constant (one branch for all of
+// a cell's slopes).  OPT: minmod.
+template <bool OPT, class F>
+__device__ __forceinline__ void with_limiter(int limiter, F f) {
+  if (OPT || limiter == 1) f(std::integral_constant<int, 1>());
+  else if (limiter == 2) f(std::integral_constant<int, 2>());
+  else f(std::integral_constant<int, 3>());
+}
+
 template <typename T>
 __device__ __forceinline__ void pred_k(const T* w, const T* s, int d, T g, T rinv, T* a) {
   if constexpr (kFast) predictor_term_fast(w, s, d, g, rinv, a);
@@ -268,21 +279,37 @@ __device__ __forceinline__ void cfl_speeds(const T* qs, const HydroParams& P, bo
   s[2] = fabs(w[3]) + a;
 }
 
+// Face states of one field with the 1D predictor (muscl.f90:68, 199-209):
+// w -+ s/2 + evo, evo = dt2 a / dx.
+template <typename T>
+__device__ __forceinline__ void faces1d(T w, T s, T dt2, T a, T dxi, T& fm, T& fp) {
+  if constexpr (kFast && sizeof(T) == 8) {
+    const T d = dt2 * a;
+    fm = fma(d, dxi, fma((T)-0.5, s, w));
+    fp = fma(d, dxi, fma((T)0.5, s, w));
+  } else {
+    const T e = dt2 * a * dxi;
+    fm = face_minus(w, s, e);
+    fp = face_plus(w, s, e);
+  }
+}
+
 // Slopes, predictor and face states of one cell.  get(f, dx, dy, dz) reads
 // primitive f of the neighbour at offset (dx, dy, dz) (one axis at a time).
 // DIM = 2 or 3 selects the 2D (muscl.f90:70-88) or 3D (89-111) predictor.
 // OPT: the usual options (minmod, second order) as constants.
 template <typename T, int DIM, bool OPT = false, typename Get>
 __device__ __forceinline__ void cell_faces_g(Get get, const HydroParams& P, T dt2, T* wv, T (*face)[2][5]) {
-  const int limiter = OPT ? 1 : P.limiter;
   T sx[5], sy[5], sz[5];
+  with_limiter<OPT>(P.limiter, [&](auto lim) {
 #pragma unroll
-  for (int f = 0; f < 5; ++f) {
-    wv[f] = get(f, 0, 0, 0);
-    sx[f] = slope_k(get(f, -1, 0, 0), wv[f], get(f, 1, 0, 0), limiter);
-    sy[f] = slope_k(get(f, 0, -1, 0), wv[f], get(f, 0, 1, 0), limiter);
-    if (DIM == 3) sz[f] = slope_k(get(f, 0, 0, -1), wv[f], get(f, 0, 0, 1), limiter);
-  }
+    for (int f = 0; f < 5; ++f) {
+      wv[f] = get(f, 0, 0, 0);
+      sx[f] = slope_k(get(f, -1, 0, 0), wv[f], get(f, 1, 0, 0), lim);
+      sy[f] = slope_k(get(f, 0, -1, 0), wv[f], get(f, 0, 1, 0), lim);
+      if (DIM == 3) sz[f] = slope_k(get(f, 0, 0, -1), wv[f], get(f, 0, 0, 1), lim);
+    }
+  });
   if (!OPT && !P.secondorder) {
     // first-order Godunov: the face states are the cell averages (sweep,
     // muscl.f90:198-201, 207-210)
@@ -299,6 +326,21 @@ __device__ __forceinline__ void cell_faces_g(Get get, const HydroParams& P, T dt
   pred_k(wv, sy, 2, g, rinv, a2);
   if (DIM == 3) pred_k(wv, sz, 3, g, rinv, a3);
   const T dxi = (T)P.dxinv, dyi = (T)P.dyinv, dzi = (T)P.dzinv;
+  if constexpr (kFast && sizeof(T) == 8) {
+    // evo = dt2 (a1 / dx + a2 / dy + a3 / dz), w -+ s/2 + evo with explicit fmas
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      T sum = fma(a2[f], dyi, a1[f] * dxi);
+      if (DIM == 3) sum = fma(a3[f], dzi, sum);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        const T s = d == 0 ? sx[f] : (d == 1 ? sy[f] : sz[f]);
+        face[d][0][f] = fma(dt2, sum, fma((T)-0.5, s, wv[f]));
+        face[d][1][f] = fma(dt2, sum, fma((T)0.5, s, wv[f]));
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int f = 0; f < 5; ++f) {
     if (DIM == 3) evo[f] = dt2 * (a1[f] * dxi + a2[f] * dyi + a3[f] * dzi);
@@ -552,7 +594,7 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<T>& A, FusedSmem<T, N
       T qo[NF];
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        qo[f] = qacc[f] + dtdz * (fz_lo[f] - fz_hi[f]);
+        qo[f] = axpy_k<kFast>(qacc[f], dtdz, fz_lo[f] - fz_hi[f]);
         A.qout[f * n + idx] = qo[f];
       }
       if (A.cfl_next) track(qo);
@@ -579,9 +621,9 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<T>& A, FusedSmem<T, N
         prim_k(qv, wdummy, c, P, de, e2);  // dual-energy resync of q (comp.f90:60-72)
       }
 #pragma unroll
-      for (int f = 0; f < NF; ++f) qv[f] = qv[f] + dtdx * (sm.fx[f][oj][oi] - sm.fx[f][oj][oi + 1]);
+      for (int f = 0; f < NF; ++f) qv[f] = axpy_k<kFast>(qv[f], dtdx, sm.fx[f][oj][oi] - sm.fx[f][oj][oi + 1]);
 #pragma unroll
-      for (int f = 0; f < NF; ++f) qacc[f] = qv[f] + dtdy * (sm.fy[f][oj][oi] - sm.fy[f][oj + 1][oi]);
+      for (int f = 0; f < NF; ++f) qacc[f] = axpy_k<kFast>(qv[f], dtdy, sm.fy[f][oj][oi] - sm.fy[f][oj + 1][oi]);
     };
 
     // prologue: planes Z0-2 .. Z0+1, B of the plane below the tile and of
@@ -732,7 +774,7 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<T>& A, FusedSmem<T, N
         T qo[NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-          qo[f] = qacc[f] + dtdz * (fz_prev[f] - fz[f]);
+          qo[f] = axpy_k<kFast>(qacc[f], dtdz, fz_prev[f] - fz[f]);
           A.qout[f * n + idx] = qo[f];
         }
         if (A.cfl_next) track(qo);
@@ -747,9 +789,9 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<T>& A, FusedSmem<T, N
           prim_k(qv, wdummy, c, P, de, e2);  // dual-energy resync of q (comp.f90:60-72)
         }
 #pragma unroll
-        for (int f = 0; f < NF; ++f) qv[f] = qv[f] + dtdx * (sm.fx[f][oj][oi] - sm.fx[f][oj][oi + 1]);
+        for (int f = 0; f < NF; ++f) qv[f] = axpy_k<kFast>(qv[f], dtdx, sm.fx[f][oj][oi] - sm.fx[f][oj][oi + 1]);
 #pragma unroll
-        for (int f = 0; f < NF; ++f) qv[f] = qv[f] + dtdy * (sm.fy[f][oj][oi] - sm.fy[f][oj + 1][oi]);
+        for (int f = 0; f < NF; ++f) qv[f] = axpy_k<kFast>(qv[f], dtdy, sm.fy[f][oj][oi] - sm.fy[f][oj + 1][oi]);
         if (DIM == 3) {
 #pragma unroll
           for (int f = 0; f < NF; ++f) qacc[f] = qv[f];
@@ -864,9 +906,7 @@ __device__ __forceinline__ void fused_cell1d(const FusedArgs<T>& A, int i) {
       pred_k(w[k + 1], s, 1, (T)P.g, kFast ? rcp_fast(w[k + 1][0]) : (T)0, a);
 #pragma unroll
       for (int f = 0; f < 5; ++f) {
-        const T e = dt2 * a[f] * dxi;
-        fm[k][f] = face_minus(w[k + 1][f], s[f], e);
-        fp[k][f] = face_plus(w[k + 1][f], s[f], e);
+        faces1d(w[k + 1][f], s[f], dt2, a[f], dxi, fm[k][f], fp[k][f]);
       }
     } else {
 #pragma unroll
@@ -884,7 +924,7 @@ __device__ __forceinline__ void fused_cell1d(const FusedArgs<T>& A, int i) {
     prim_k(qv, wd, c, P, de, e2);
   }
 #pragma unroll
-  for (int f = 0; f < NF; ++f) A.qout[f * n + i] = qv[f] + dtdx * (flo[f] - fhi[f]);
+  for (int f = 0; f < NF; ++f) A.qout[f * n + i] = axpy_k<kFast>(qv[f], dtdx, flo[f] - fhi[f]);
   if (err) {
 #if defined(EVORA_HOST_EMU)
     reinterpret_cast<std::atomic<unsigned>*>(&A.ctl->err)->fetch_or(err);

@@ -117,7 +117,7 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
         T qo[NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-          qo[f] = qacc[f] + dtdy * (fy[f] - fn[f]);
+          qo[f] = axpy_k<kFast>(qacc[f], dtdy, fy[f] - fn[f]);
           A.qout[f * n + idx] = qo[f];
         }
         if (A.cfl_next) {
@@ -145,7 +145,7 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
       }
 #pragma unroll
       for (int f = 0; f < NF; ++f)
-        qacc[f] = qc[f] + dtdx * (fx[f] - __shfl_down_sync(0xffffffffu, fx[f], 1));
+        qacc[f] = axpy_k<kFast>(qc[f], dtdx, fx[f] - __shfl_down_sync(0xffffffffu, fx[f], 1));
     }
 #pragma unroll
     for (int f = 0; f < 5; ++f) {

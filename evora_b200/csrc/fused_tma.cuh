@@ -422,7 +422,7 @@ __device__ __forceinline__ void tma_tile(const FusedArgs<T>& A, const TmaMap& ma
     T qo[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
-      qo[f] = qacc[f] + dtdz * (fz_lo[f] - fz_hi[f]);
+      qo[f] = axpy_k<kFast>(qacc[f], dtdz, fz_lo[f] - fz_hi[f]);
       A.qout[f * n + idx] = qo[f];
     }
     if (A.cfl_next) {
@@ -455,9 +455,9 @@ __device__ __forceinline__ void tma_tile(const FusedArgs<T>& A, const TmaMap& ma
       prim_k(qv, wdummy, c, P, de, e2);   // dual-energy resync of q (comp.f90:60-72)
     }
 #pragma unroll
-    for (int f = 0; f < NF; ++f) qv[f] = qv[f] + dtdx * (sm.fx[f][oj][oi] - sm.fx[f][oj][oi + 1]);
+    for (int f = 0; f < NF; ++f) qv[f] = axpy_k<kFast>(qv[f], dtdx, sm.fx[f][oj][oi] - sm.fx[f][oj][oi + 1]);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) qacc[f] = qv[f] + dtdy * (sm.fy[f][oj][oi] - sm.fy[f][oj + 1][oi]);
+    for (int f = 0; f < NF; ++f) qacc[f] = axpy_k<kFast>(qv[f], dtdy, sm.fy[f][oj][oi] - sm.fy[f][oj + 1][oi]);
   };
 
   T* const ring0 = &sm.w[0][0][0][0];

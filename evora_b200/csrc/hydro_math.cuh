@@ -425,53 +425,84 @@ __device__ __forceinline__ T minmod_fast(T dwl, T dwr) {
   return dwl * dwr > (T)0 ? copysign(m, dwl) : (T)0;
 }
 
+// The other limiters (muscl.f90:141-163) in the fast form: the monotonised
+// central one without branches (the central difference has the sign the two
+// others share), van Leer's with the fast reciprocal in FP64.
 template <typename T>
 __device__ __forceinline__ T slope_fast(T wl, T w, T wr, int limiter) {
-  if (limiter == 1) return minmod_fast(w - wl, wr - w);
-  return slope1(wl, w, wr, limiter);
+  const T dwl = w - wl, dwr = wr - w;
+  if (limiter == 1) return minmod_fast(dwl, dwr);
+  if (limiter == 2) {
+    const T dwc = (wr - wl) * (T)0.5;
+    const T m = fmin(fmin((T)2.0 * fabs(dwl), fabs(dwc)), (T)2.0 * fabs(dwr));
+    return dwl * dwr > (T)0 ? copysign(m, dwl) : (T)0;
+  }
+  if constexpr (sizeof(T) == 8) {
+    const T pro = dwl * dwr;
+    return pro > (T)0 ? (T)2.0 * pro * rcp_fast(dwr + dwl) : (T)0;
+  } else {
+    return slope1(wl, w, wr, 3);
+  }
 }
+
+// The FP64 fast forms write every sum that takes a product as an explicit
+// fma, so that no choice of contraction is left to the compiler: it differs
+// between instantiations of a kernel, and tile shapes, grids and batches would
+// then agree to a few ulp only.
+__device__ __forceinline__ double mul_rn(double a, double b) {   // a product that no sum takes in
+#if defined(__CUDA_ARCH__)
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+__device__ __forceinline__ double sq3(double a, double b, double c) { return fma(c, c, fma(b, b, a * a)); }
 
 // q2w with dual energy (comp.f90:26-43, 45-85) in the fast forms: one
 // reciprocal of rho, the kin/E switch as kin * (1/E), rho^(g-1) by
 // pow_fast; resynchronises E (S system) or S (E system) in q as pressure()
 // does.
-template <typename T>
-__device__ __forceinline__ void q2w_de_fast(T* q, T* w, const Gas<T>& c, unsigned& err) {
-  const T densinv = rcp_fast(q[0]);
+__device__ __forceinline__ void q2w_de_fast(double* q, double* w, const Gas<double>& c, unsigned& err) {
+  const double densinv = rcp_fast(q[0]);
   w[0] = q[0];
-  w[1] = q[1] * densinv;
-  w[2] = q[2] * densinv;
-  w[3] = q[3] * densinv;
-  const T m2 = (q[1] * q[1]) + (q[2] * q[2]) + (q[3] * q[3]);
-  const T kin = (T)0.5 * m2 * densinv;
-  const T pg = pow_fast(q[0], c.g1);
-  T press;
+  w[1] = mul_rn(q[1], densinv);
+  w[2] = mul_rn(q[2], densinv);
+  w[3] = mul_rn(q[3], densinv);
+  const double hm2 = 0.5 * sq3(q[1], q[2], q[3]);
+  const double kin = mul_rn(hm2, densinv);
+  const double pg = pow_fast(q[0], c.g1);
+  double press;
   if (kin * rcp_fast(q[4]) > c.de_thresh1) {
-    press = q[5] * pg;
-    q[4] = kin + press * c.g1inv;
+    press = mul_rn(q[5], pg);
+    q[4] = fma(press, c.g1inv, kin);
   } else {
-    press = c.g1 * (q[4] - kin);
-    q[5] = press * rcp_fast(pg);
+    press = mul_rn(c.g1, q[4] - kin);
+    q[5] = mul_rn(press, rcp_fast(pg));
   }
-  if (press <= (T)0) err |= EVORA_ERR_PRESSURE;
+  if (press <= 0.0) err |= EVORA_ERR_PRESSURE;
   w[4] = press;
 }
 
 // q2w with one reciprocal (comp.f90:26-43, 56-71 without dual energy).
-template <typename T>
-__device__ __forceinline__ void q2w_fast(const T* q, T* w, const Gas<T>& c, unsigned& err) {
-  const T densinv = rcp_fast(q[0]);
+__device__ __forceinline__ void q2w_fast(const double* q, double* w, const Gas<double>& c, unsigned& err) {
+  const double densinv = rcp_fast(q[0]);
   w[0] = q[0];
-  w[1] = q[1] * densinv;
-  w[2] = q[2] * densinv;
-  w[3] = q[3] * densinv;
-  const T m2 = (q[1] * q[1]) + (q[2] * q[2]) + (q[3] * q[3]);
-  const T p = c.g1 * (q[4] - (T)0.5 * m2 * densinv);
-  if (p <= (T)0) err |= EVORA_ERR_PRESSURE;
+  w[1] = mul_rn(q[1], densinv);
+  w[2] = mul_rn(q[2], densinv);
+  w[3] = mul_rn(q[3], densinv);
+  const double p = mul_rn(c.g1, fma(-0.5 * sq3(q[1], q[2], q[3]), densinv, q[4]));
+  if (p <= 0.0) err |= EVORA_ERR_PRESSURE;
   w[4] = p;
 }
 
 // predictor term with the 1/rho of the cell given (muscl.f90:100-104).
+__device__ __forceinline__ void predictor_term_fast(const double* w, const double* s, int d, double g, double rinv,
+                                                    double* a) {
+#pragma unroll
+  for (int f = 0; f < 5; ++f) a[f] = w[d] * s[f];
+  a[4] = fma(g * w[4], s[d], a[4]);
+  a[d] = fma(s[4], rinv, a[d]);
+}
 template <typename T>
 __device__ __forceinline__ void predictor_term_fast(const T* w, const T* s, int d, T g, T rinv, T* a) {
 #pragma unroll
@@ -481,8 +512,56 @@ __device__ __forceinline__ void predictor_term_fast(const T* w, const T* s, int 
 }
 
 // HLLC (riemann.f90:96-153) in the fast form.  DIR = 1..3.
+template <int NF, int DIR>
+__device__ __forceinline__ void hllc_fast64(const double* wl, const double* wr, double* f, const Gas<double>& c,
+                                            unsigned& err) {
+  if (wl[4] <= 0.0 || wr[4] <= 0.0) err |= EVORA_ERR_RIEMANN_PRESSURE;
+  const double ril = rcp_fast(wl[0]), rir = rcp_fast(wr[0]);
+  const double al = sqrt_fast(c.g * wl[4] * ril);
+  const double ar = sqrt_fast(c.g * wr[4] * rir);
+  const double ul = wl[DIR], ur = wr[DIR];
+  const double sl = fmin2(ul - al, ur - ar);
+  const double sr = fmax2(ul + al, ur + ar);
+  const double dl = sl - ul;
+  const double facl = wl[0] * dl;
+  const double facr = wr[0] * (sr - ur);
+  const double sm = mul_rn(fma(-facr, ur, fma(facl, ul, wr[4] - wl[4])), rcp_fast(fma(wl[0], dl, -facr)));
+  const bool pure_left = 0.0 <= sl;
+  const bool pure_right = !pure_left && 0.0 >= sr;
+  const bool star = !pure_left && !pure_right;
+  const bool left = pure_left || (star && 0.0 < sm);
+  if (!(sl == sl && sr == sr && sm == sm)) err |= EVORA_ERR_HLLC;
+  double w[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) w[i] = left ? wl[i] : wr[i];
+  const double ri = left ? ril : rir;
+  const double sk = left ? sl : sr;
+  const double fk = left ? facl : facr;
+  const double ud = w[DIR];
+  const double e = fma(0.5 * w[0], sq3(w[1], w[2], w[3]), w[4] * c.g1inv);   // total energy
+  const double mu = w[0] * ud;                                                // mass flux
+  // the plain flux fl and, with the star state qx (statex, riemann.f90:241-288),
+  // fl + sk (qx - ql); the transverse momenta (and the entropy) of either are
+  // the mass flux times the side's velocity (p / rho^g)
+  const double rc = rcp_fast(sk - sm);
+  const double chi = fk * rc;                      // rho (s - u_d) / (s - sm)
+  const double ex = fma(sm - ud, fma(w[4], rcp_fast(fk), sm), e * ri);
+  const double f0 = star ? fma(sk, fma(fk, rc, -w[0]), mu) : mu;
+  const double fd = fma(mu, ud, star ? fma(sk, fma(chi, sm, -mu), w[4]) : w[4]);
+  const double fe = fma(ud, e + w[4], star ? sk * fma(chi, ex, -e) : 0.0);
+  f[0] = f0;
+#pragma unroll
+  for (int i = 1; i < 4; ++i) f[i] = i == DIR ? fd : mul_rn(f0, w[i]);
+  f[4] = fe;
+  if (NF == 6) f[5] = mul_rn(f0 * ri, w[4] * rcp_fast(pow_fast(w[0], c.g1)));
+}
+
 template <typename T, int NF, int DIR>
 __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const Gas<T>& c, unsigned& err) {
+  if constexpr (sizeof(T) == 8) {
+    hllc_fast64<NF, DIR>(wl, wr, f, c, err);
+    return;
+  }
   if (wl[4] <= (T)0 || wr[4] <= (T)0) err |= EVORA_ERR_RIEMANN_PRESSURE;
   const T ril = rcp_fast(wl[0]), rir = rcp_fast(wr[0]);
   const T al = sqrt_fast(c.g * wl[4] * ril);
@@ -547,11 +626,67 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   for (int i = 0; i < NF; ++i) f[i] = fl[i] + sk * (qx[i] - ql[i]);
 }
 
+// HLL (riemann.f90:47-92) in the fast form, FP64: with the speeds clamped to
+// sl <= 0 <= sr the star formula gives the plain left (right) flux where all
+// waves go right (left), so there is no branch and one reciprocal of sr - sl
+// instead of NF divisions.  333 x 250 cells FP64, HLL and moncen, with the
+// limiter's fast form: 22.5 -> 16.1 us per step.
+template <int NF, int DIR>
+__device__ __forceinline__ void hll_fast(const double* wl, const double* wr, double* f, const Gas<double>& c,
+                                         unsigned& err) {
+  if (wl[4] <= 0.0 || wr[4] <= 0.0) err |= EVORA_ERR_RIEMANN_PRESSURE;
+  const double al = sqrt_fast(c.g * wl[4] * rcp_fast(wl[0]));
+  const double ar = sqrt_fast(c.g * wr[4] * rcp_fast(wr[0]));
+  const double ul = wl[DIR], ur = wr[DIR];
+  double sl = fmin2(ul - al, ur - ar), sr = fmax2(ul + al, ur + ar);
+  if (!(sl == sl && sr == sr)) err |= EVORA_ERR_HLL;
+  sl = fmin2(sl, 0.0);
+  sr = fmax2(sr, 0.0);
+  const double inv = rcp_fast(sr - sl);
+  const double a = sr * inv, b = -sl * inv, ab = sl * a;   // f = a fl + b fr + sl sr / (sr - sl) (qr - ql)
+  double q[2][6], fl[2][6];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double* w = k ? wr : wl;
+    const double ud = w[DIR];
+    const double e = fma(0.5 * w[0], sq3(w[1], w[2], w[3]), w[4] * c.g1inv);
+    const double mu = w[0] * ud;
+    q[k][0] = w[0];
+    fl[k][0] = mu;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      q[k][i] = w[0] * w[i];
+      fl[k][i] = mu * w[i];
+    }
+    fl[k][DIR] = fma(mu, ud, w[4]);
+    q[k][4] = e;
+    fl[k][4] = ud * (e + w[4]);
+    if (NF == 6) {
+      const double s = w[4] * rcp_fast(pow_fast(w[0], c.g1));
+      q[k][5] = s;
+      fl[k][5] = ud * s;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NF; ++i) f[i] = fma(ab, q[1][i], fma(-ab, q[0][i], fma(b, fl[1][i], a * fl[0][i])));
+}
+
 template <typename T, int NF, int DIR>
 __device__ __forceinline__ void riemann_fast(const T* wl, const T* wr, T* f, int solver, const Gas<T>& c,
                                              unsigned& err) {
-  if (solver == 2) hllc_fast<T, NF, DIR>(wl, wr, f, c, err);
-  else hll<T, NF>(wl, wr, f, DIR, c, err);
+  if (solver == 2) {
+    hllc_fast<T, NF, DIR>(wl, wr, f, c, err);
+  } else {
+    if constexpr (sizeof(T) == 8) hll_fast<NF, DIR>(wl, wr, f, c, err);
+    else hll<T, NF>(wl, wr, f, DIR, c, err);
+  }
+}
+
+// x + a b: an explicit fma in the FP64 fast forms (FAST), else left as written.
+template <bool FAST, typename T>
+__device__ __forceinline__ T axpy_k(T x, T a, T b) {
+  if constexpr (FAST && sizeof(T) == 8) return fma(a, b, x);
+  else return x + a * b;
 }
 
 // Interface states of sweep (muscl.f90:199-200, 208-209): the state a cell
