@@ -18,7 +18,8 @@ int chem_step(const HydroParams& P, void* q, bool f32, int nf, int64_t n, double
 // sub-cycle (shared powers of T, a table-driven exponential, contracted
 // products), within a few ulp of chem_step per rate (chem_fast.cu).  With
 // expand, each cell then takes the expansion terms of a comoving run
-// (expansion(q), cosmology.f90:53-72) in the same pass.
+// (expansion(q), cosmology.f90:53-72) in the same pass.  The next step's CFL
+// maxima of the state it writes go to ctl->snext.
 int chem_step_fast(const HydroParams& P, void* q, bool f32, int nf, int64_t n, double* species, GridCtl* ctl,
                    cudaStream_t st, bool expand = false);
 

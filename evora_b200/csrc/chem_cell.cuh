@@ -1,7 +1,7 @@
 // chem_cell.cuh -- one cell of chem(q) (chemistry.f90:72-121) and the
-// per-cell loop of the resident SoA kernel, shared by the reference-order
-// kernels (chem.cu, compiled without FMA contraction) and the reduced-work
-// ones of the default mode (chem_fast.cu).  The CIE update is a policy:
+// per-cell loop of the resident SoA kernel, of the reference-order kernels
+// (chem.cu, compiled without FMA contraction); the default mode's kernel has
+// its own (chem_fast.cu).  The CIE update is a policy:
 // Cie::run(C, k, temp0, dt, rho, press, n, err) does cie (cie.f90:26-56).
 //
 //   press = pressure(q)                              (dual-energy write-back)
@@ -51,31 +51,18 @@ __device__ __forceinline__ void chem_cell(double* v, double* n, const HydroParam
   }
 }
 
-// The expansion terms of a comoving run (expansion(q), cosmology.f90:53-72)
-// on the same cell, kx = dt g35 expand: press = pressure(q) (write-back),
-// E -= kx press / g1, S -= kx S.
-template <class Cie>
-__device__ __forceinline__ void expand_cell_t(double* v, double kx, const HydroParams& P, const Gas<double>& c,
-                                              const Cie& cie_fn, unsigned& err) {
-  const double press = cie_fn.pressure(v, c, P.dualenergy != 0, err);
-  v[4] = v[4] - cie_fn.div(kx * press, P.g1, P.g1inv);
-  v[5] = v[5] - kx * v[5];
-}
-
 // chem(q) over the cells of a SoA state q (nf fields of n cells, T = float
 // or double) with its FP64 species (kNs field-major arrays), grid-stride;
 // errors OR-ed into *err.  S (field 5) is not carried when nf = 5: its
-// terms are dropped.  expand: the expansion terms follow on each cell
-// (main.f90:178 runs them right after chem when there is no conduction).
+// terms are dropped.
 template <typename T, class Cie>
 __device__ __forceinline__ void chem_soa(T* __restrict__ q, int64_t n, int nf, double* __restrict__ species,
                                          const HydroParams& P, const GridCtl* ctl, const Cie& cie_fn,
-                                         unsigned* err, bool expand = false) {
+                                         unsigned* err) {
   const Gas<double> c = Gas<double>::make(P);
   const Units U = units_of(P, ctl);
   const ChemCoef& k = ctl->coef;
   const double dt = ctl->dt;
-  const double kx = dt * P.g35 * ctl->expand;
   unsigned e = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double v[6], s[kNs];
@@ -84,7 +71,6 @@ __device__ __forceinline__ void chem_soa(T* __restrict__ q, int64_t n, int nf, d
 #pragma unroll
       for (int j = 0; j < kNs; ++j) s[j] = species[j * n + i];
     chem_cell(v, s, P, U, k, dt, c, cie_fn, e);
-    if (expand) expand_cell_t(v, kx, P, c, cie_fn, e);
     q[4 * n + i] = (T)v[4];
     if (nf == 6) q[5 * n + i] = (T)v[5];
     if (P.chemistry)
@@ -106,8 +92,6 @@ struct CieExact {
   }
   // a / x^y
   __device__ __forceinline__ double div_pow(double a, double x, double y) const { return a / pow(x, y); }
-  // a / b (binv = 1/b rounded, unused)
-  __device__ __forceinline__ double div(double a, double b, double) const { return a / b; }
 };
 
 }  // namespace evora

@@ -1,5 +1,5 @@
 // chem_fast.cu -- chem(q) (chemistry.f90:72-121) of the default (not
-// STRICT) mode on a resident SoA state: the cell update of chem_cell.cuh with
+// STRICT) mode on a resident SoA state: the cell update of chem_cell.cuh, with
 // the CIE cooling sub-cycles (cie.f90:26-56) evaluating fewer FP64
 // operations per cycle than the reference's order of operations (chem.cu):
 //
@@ -28,8 +28,8 @@
 #include <cstdint>
 
 #include "../../include/evora_gpu.h"
+#include "cfl_reduce.cuh"
 #include "chem.h"
-#include "chem_cell.cuh"
 #include "chemistry.cuh"
 #include "common.h"
 #include "fast_exp.cuh"
@@ -164,30 +164,6 @@ template <class Exp, class Coef>
 struct CieFast {
   Exp ex;
   Coef kc;
-  // pressure() (comp.f90:45-85) with the fast forms: kin/E as kin (1/E),
-  // rho^(g-1) = exp((g-1) ln rho), the divisions as products with
-  // reciprocals; the same write-back of E or S
-  __device__ __forceinline__ double pressure(double* q, const Gas<double>& c, bool de, unsigned& err) const {
-    const double m2 = (q[1] * q[1]) + (q[2] * q[2]) + (q[3] * q[3]);
-    const double kin = 0.5 * m2 * rcp64(q[0]);
-    double press;
-    if (de) {
-      const double pg = ex(c.g1 * log(q[0]));
-      if (kin * rcp64(q[4]) > c.de_thresh1) {
-        press = q[5] * pg;
-        q[4] = kin + press * c.g1inv;
-      } else {
-        press = c.g1 * (q[4] - kin);
-        q[5] = press * rcp64(pg);
-      }
-    } else {
-      press = c.g1 * (q[4] - kin);
-    }
-    if (press <= 0.0) err |= EVORA_ERR_PRESSURE;
-    return press;
-  }
-  __device__ __forceinline__ double div_pow(double a, double x, double y) const { return a * rcp64(ex(y * log(x))); }
-  __device__ __forceinline__ double div(double a, double, double binv) const { return a * binv; }
   __device__ __forceinline__ void run(const ChemParams& C, const ChemCoef& k, double temp0, double dt, double rho,
                                       double& press, double* n, unsigned& err) const {
     const double nH = C.chiH * rho, nHe = C.chiHe * rho;
@@ -236,23 +212,91 @@ struct CieFast {
   }
 };
 
-// chem(q) on the resident SoA state, with Tang's exponential (its table
-// staged in shared memory) and the rate coefficients read from shared
-// memory where they are used.  Both measured faster in the 256^3
-// cosmological box: with the library's exp the kernel ran about 14 % slower,
-// with the coefficients in registers about 5 %.  expand: the expansion
-// terms in the same pass.
+// One cell's pressure() (comp.f90:45-85) in the fast forms, with its
+// write-back of E or S; kin its kinetic energy, pg = rho^(g-1).
+__device__ __forceinline__ double pressure_of(double* v, double kin, double pg, const HydroParams& P, unsigned& err) {
+  double press = P.g1 * (v[4] - kin);
+  if (P.dualenergy) {
+    if (kin * rcp64(v[4]) > P.de_thresh1) {
+      press = v[5] * pg;
+      v[4] = kin + press * P.g1inv;
+    } else {
+      v[5] = press * rcp64(pg);
+    }
+  }
+  if (press <= 0.0) err |= EVORA_ERR_PRESSURE;
+  return press;
+}
+
+// chem(q) on the resident SoA state (the steps of chem_cell.cuh), with
+// Tang's exponential (its table staged in shared memory) and the rate
+// coefficients read from shared memory where they are used.  Both measured
+// faster in the 256^3 cosmological box: with the library's exp the kernel ran
+// about 14 % slower, with the coefficients in registers about 5 %.  expand:
+// the expansion terms in the same pass (main.f90:178 runs them right after
+// chem when there is no conduction).  As this is the step's last pass over the
+// state it also reduces the next step's CFL maxima.  rho and the momenta do
+// not change in here, so the kinetic energy and rho^(g-1) are formed once for
+// the pressure recoveries before and after the cooling and for the maxima.
 template <typename T, int MINB>
 __global__ void __launch_bounds__(kChemThreads, MINB)
-k_chem_fast(T* __restrict__ q, int64_t n, int nf, double* __restrict__ species, HydroParams P, const GridCtl* ctl,
-            unsigned* err, bool expand) {
+k_chem_fast(T* __restrict__ q, int64_t n, int nf, double* __restrict__ species, HydroParams P, GridCtl* ctl,
+            bool expand) {
   if (ctl_skip(ctl)) return;
   __shared__ double tab[32];
   __shared__ double coef[2 * kNcool];
+  __shared__ double red[3][32];
   if (threadIdx.x < 32) tab[threadIdx.x] = kExp2Frac[threadIdx.x];
   if (threadIdx.x < 2 * kNcool) coef[threadIdx.x] = ctl->coef.c[threadIdx.x >> 1][threadIdx.x & 1];
   __syncthreads();
-  chem_soa(q, n, nf, species, P, ctl, CieFast<ExpTable, CoefShared>{ExpTable{tab}, CoefShared{coef}}, err, expand);
+  const CieFast<ExpTable, CoefShared> cie{ExpTable{tab}, CoefShared{coef}};
+  const Gas<double> c = Gas<double>::make(P);
+  const Units U = units_of(P, ctl);
+  const double dt = ctl->dt;
+  const double kx = dt * P.g35 * ctl->expand;
+  unsigned e = 0;
+  CflEpilogue<T, true> cfl;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double v[6], s[kNs];
+    load_cell(q, n, nf, i, v);
+    if (P.chemistry)
+#pragma unroll
+      for (int j = 0; j < kNs; ++j) s[j] = species[j * n + i];
+    const double kin = 0.5 * ((v[1] * v[1]) + (v[2] * v[2]) + (v[3] * v[3])) * rcp64(v[0]);
+    const double pg = nf == 6 ? cie.ex(P.g1 * log(v[0])) : 1.0;
+    double press = pressure_of(v, kin, pg, P, e);
+    const double oldpress = press;
+    if (P.chemistry) {
+      const ChemParams C{P.cooling, P.background, P.chiH, P.chiHe, P.c_chem, P.substep};
+      cie.run(C, ctl->coef, U.temp0, dt, v[0], press, s, e);
+    }
+    if (P.cooling || P.tempfloor || P.jeansfloor) {
+      if (P.tempfloor) {
+        const double pfloor = P.temp_fl * (P.chemistry ? nsum(s) : v[0]) * U.temp0inv;
+        if (pfloor > press) press = pfloor;
+      }
+      if (P.jeansfloor) {
+        const double pfloor = P.jeansfloor0 * v[0] * v[0];
+        if (pfloor > press) press = pfloor;
+      }
+      const double dpress = press - oldpress;
+      v[4] = v[4] + dpress * P.g1inv;
+      v[5] = v[5] + dpress * rcp64(pg);
+    }
+    if (expand) {
+      press = pressure_of(v, kin, pg, P, e);
+      v[4] = v[4] - kx * press * P.g1inv;
+      v[5] = v[5] - kx * v[5];
+    }
+    q[4 * n + i] = (T)v[4];
+    if (nf == 6) q[5 * n + i] = (T)v[5];
+    if (P.chemistry)
+#pragma unroll
+      for (int j = 0; j < kNs; ++j) species[j * n + i] = s[j];
+    cfl.add(v, pg, P, c);
+  }
+  if (e) atomicOr(&ctl->err, e);
+  cfl.finish(ctl, red);
 }
 
 // The self-test of the error bounds over x[0..n): out[i] = Tang's exp(x[i]),
@@ -281,10 +325,10 @@ int chem_step_fast(const HydroParams& P, void* q, bool f32, int nf, int64_t n, d
   const int blocks = (int)(want < cap ? (want < 1 ? 1 : want) : cap);
   if (f32)
     k_chem_fast<float, kChemMinBlocks>
-        <<<blocks, kChemThreads, 0, st>>>((float*)q, n, nf, species, P, ctl, &ctl->err, expand);
+        <<<blocks, kChemThreads, 0, st>>>((float*)q, n, nf, species, P, ctl, expand);
   else
     k_chem_fast<double, kChemMinBlocks>
-        <<<blocks, kChemThreads, 0, st>>>((double*)q, n, nf, species, P, ctl, &ctl->err, expand);
+        <<<blocks, kChemThreads, 0, st>>>((double*)q, n, nf, species, P, ctl, expand);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_cuda_error(e, "chem");

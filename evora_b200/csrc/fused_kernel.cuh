@@ -36,6 +36,9 @@
 #include <type_traits>
 
 #include "hydro_math.cuh"
+#if !defined(EVORA_HOST_EMU)
+#include "cfl_reduce.cuh"
+#endif
 
 #ifdef EVORA_HOST_EMU
 #include <algorithm>
@@ -935,20 +938,6 @@ __device__ __forceinline__ void fused_cell1d(const FusedArgs<T>& A, int i) {
 }
 
 #if !defined(EVORA_HOST_EMU)
-// The largest of a non-negative value (no NaN) over a warp, or over red[0..NW)
-// for every lane: values >= 0 order like their bits, which one (FP32) or two
-// (FP64: high words, then the low words of those that have the largest)
-// warp reductions of unsigned words take.
-__device__ __forceinline__ float warp_max_pos(float v) {
-  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
-}
-__device__ __forceinline__ double warp_max_pos(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
-  return __hiloint2double((int)mh, (int)ml);
-}
-
 // The step control after a hydro-only 2D update (no physics, not comoving), by
 // the last CTA to finish: A.tail = 1 the step's end, and the next step's
 // begin and time from the maxima this update reduced (k_step_control's work,

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/evora_gpu.h"
+#include "cfl_reduce.cuh"
 #include "common.h"
 #include "cosmology.cuh"
 #include "gravity.h"
@@ -124,17 +125,21 @@ __global__ void k_green(cufftDoubleComplex* __restrict__ spec, int nxh, int ny, 
 // the cell's expansion terms follow in the same pass: pressure() of the
 // updated cell, E -= dt g35 expand p / g1, S -= dt g35 expand S -- the same
 // per-cell arithmetic as the separate pass, without its trip through HBM.
-template <typename T, bool EXPAND>
+// CFL: the next step's maxima are reduced from the cells it writes
+// (cfl_reduce.cuh), in the literal (1) or the fast forms (2); 0: not.
+template <typename T, bool EXPAND, int CFL>
 __global__ void k_integrate(T* __restrict__ q, int64_t n, int nf, int aos, const double* __restrict__ phi, int nx,
-                            int ny, int nz, double dx2inv, double dy2inv, double dz2inv, const GridCtl* ctl,
+                            int ny, int nz, double dx2inv, double dy2inv, double dz2inv, GridCtl* ctl,
                             double dt_host, HydroParams P) {
   // (the entropy field, when carried, is not touched by gravintegration:
   // it updates E and m only)
   // 3D launch: x by threads, one (y, z) row per block row
+  __shared__ double red[3][32];
   if (ctl_skip(ctl)) return;
   const double dt = ctl ? ctl->dt : dt_host;
   const int64_t nxy = (int64_t)nx * ny;
   const int ix = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y, iz = blockIdx.z;
+  CflEpilogue<T, CFL == 2> cfl;
   if (ix < nx) {
     const int64_t i = ((int64_t)iz * ny + iy) * nx + ix;
     double f1 = 0.0, f2 = 0.0, f3 = 0.0;
@@ -153,27 +158,48 @@ __global__ void k_integrate(T* __restrict__ q, int64_t n, int nf, int aos, const
     double v[6];
 #pragma unroll
     for (int f = 0; f < 5; ++f) v[f] = aos ? (double)q[6 * i + f] : (double)q[f * n + i];
+    // S is 0 when not carried (and read only for grid states)
+    v[5] = (EXPAND || CFL) && nf == 6 ? (double)q[5 * n + i] : 0.0;
     v[4] = v[4] + dt * (v[1] * f1 + v[2] * f2 + v[3] * f3);
     v[1] = v[1] + dt * v[0] * f1;
     v[2] = v[2] + dt * v[0] * f2;
     v[3] = v[3] + dt * v[0] * f3;
+    double pg = 0.0;   // rho^(g-1)
+    if (CFL == 2 && P.dualenergy) pg = pow_fast(v[0], P.g1);
     if (EXPAND) {
-      // grid states only (aos = 0); S is 0 when not carried
-      v[5] = nf == 6 ? (double)q[5 * n + i] : 0.0;
-      unsigned err = 0;
-      const double press = pressure(v, Gas<double>::make(P), P.dualenergy != 0, err);
+      // grid states only (aos = 0)
       const double k = dt * P.g35 * ctl->expand;
-      v[4] = v[4] - k * press / P.g1;
+      unsigned err = 0;
+      if constexpr (CFL == 2) {
+        // pressure() in the fast forms, with its write-back
+        const double kin = 0.5 * sq3(v[1], v[2], v[3]) * rcp_fast(v[0]);
+        double press = P.g1 * (v[4] - kin);
+        if (P.dualenergy) {
+          if (kin * rcp_fast(v[4]) > P.de_thresh1) {
+            press = v[5] * pg;
+            v[4] = kin + press * P.g1inv;
+          } else {
+            v[5] = press * rcp_fast(pg);
+          }
+        }
+        if (press <= 0.0) err |= EVORA_ERR_PRESSURE;
+        v[4] = v[4] - k * press * P.g1inv;
+      } else {
+        const double press = pressure(v, Gas<double>::make(P), P.dualenergy != 0, err);
+        v[4] = v[4] - k * press / P.g1;
+      }
       v[5] = v[5] - k * v[5];
       if (nf == 6) q[5 * n + i] = (T)v[5];
-      if (err) atomicOr(const_cast<unsigned*>(&ctl->err), err);
+      if (err) atomicOr(&ctl->err, err);
     }
 #pragma unroll
     for (int f = 1; f < 5; ++f) {
       if (aos) q[6 * i + f] = (T)v[f];
       else q[f * n + i] = (T)v[f];
     }
+    if (CFL) cfl.add(v, pg, P, Gas<double>::make(P));
   }
+  if (CFL) cfl.finish(ctl, red);
 }
 
 }  // namespace
@@ -304,21 +330,25 @@ int grav_potential(GravPlan& g, const void* q, bool f32, int nf, int aos, const 
   return 0;
 }
 
-int grav_integrate(GravPlan& g, void* q, bool f32, int nf, int aos, const GridCtl* ctl, double dt_host,
-                   const HydroParams* expand) {
-  cudaStream_t st = g.stream;
+namespace {
+template <typename T>
+void launch_integrate(GravPlan& g, void* q, int nf, int aos, GridCtl* ctl, double dt_host, const HydroParams& P,
+                      bool expand, int cfl) {
   const dim3 rows((g.nx + kRow - 1) / kRow, g.ny, g.nz);
-  if (expand && (aos || !ctl)) return EVORA_ERR_ARG;   // the fused expansion reads dt, expand from a grid
-  const HydroParams P = expand ? *expand : HydroParams{};
-  if (f32) {
-    auto k = expand ? k_integrate<float, true> : k_integrate<float, false>;
-    k<<<rows, kRow, 0, st>>>((float*)q, g.n, nf, aos, g.phi, g.nx, g.ny, g.nz, g.dx2inv, g.dy2inv, g.dz2inv, ctl,
-                             dt_host, P);
-  } else {
-    auto k = expand ? k_integrate<double, true> : k_integrate<double, false>;
-    k<<<rows, kRow, 0, st>>>((double*)q, g.n, nf, aos, g.phi, g.nx, g.ny, g.nz, g.dx2inv, g.dy2inv, g.dz2inv, ctl,
-                             dt_host, P);
-  }
+  auto k = k_integrate<T, false, 0>;
+  if (expand) k = cfl == 2 ? k_integrate<T, true, 2> : (cfl == 1 ? k_integrate<T, true, 1> : k_integrate<T, true, 0>);
+  else if (cfl) k = cfl == 2 ? k_integrate<T, false, 2> : k_integrate<T, false, 1>;
+  k<<<rows, kRow, 0, g.stream>>>((T*)q, g.n, nf, aos, g.phi, g.nx, g.ny, g.nz, g.dx2inv, g.dy2inv, g.dz2inv, ctl,
+                                 dt_host, P);
+}
+}  // namespace
+
+int grav_integrate(GravPlan& g, void* q, bool f32, int nf, int aos, GridCtl* ctl, double dt_host,
+                   const HydroParams* grid, bool expand, int cfl) {
+  if ((expand || cfl) && (aos || !ctl || !grid)) return EVORA_ERR_ARG;   // they run on a grid's state
+  const HydroParams P = grid ? *grid : HydroParams{};
+  if (f32) launch_integrate<float>(g, q, nf, aos, ctl, dt_host, P, expand, cfl);
+  else launch_integrate<double>(g, q, nf, aos, ctl, dt_host, P, expand, cfl);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_cuda_error(e, "gravintegration");

@@ -44,10 +44,12 @@ int grav_potential(GravPlan& g, const void* q, bool f32, int nf, int aos, const 
 
 // gravintegration (gravitation.f90:170-194) with the forces of grav_force
 // (196-243), in place on the state, with the step's dt from ctl (or dt_host
-// when ctl is null).  With `expand` (a grid's parameters; SoA state and ctl
-// required) the comoving step's expansion terms (cosmology.f90:53-72) are
-// applied to each cell in the same pass.
-int grav_integrate(GravPlan& g, void* q, bool f32, int nf, int aos, const GridCtl* ctl, double dt_host,
-                   const HydroParams* expand = nullptr);
+// when ctl is null).  On a grid (its parameters in `grid`; SoA state and ctl
+// required), with `expand` the comoving step's expansion terms
+// (cosmology.f90:53-72) are applied to each cell in the same pass, and with
+// `cfl` the next step's CFL maxima are reduced from the cells written: 1 in
+// the literal, 2 in the fast forms.
+int grav_integrate(GravPlan& g, void* q, bool f32, int nf, int aos, GridCtl* ctl, double dt_host,
+                   const HydroParams* grid = nullptr, bool expand = false, int cfl = 0);
 
 }  // namespace evora

@@ -135,6 +135,10 @@ size_t elem_size(const evora_grid* g) { return g->precision == EVORA_FP32 ? 4 : 
 // kernel fills smax after this; 2: a CFL kernel filled smax before this.
 __device__ __forceinline__ void step_begin(GridCtl* ctl, int use_next) {
   if (use_next == 1) {
+    if (ctl->dump != 0) {   // a held step leaves the maxima to the step after the hold
+      ctl->active = 0;
+      return;
+    }
     ctl->err |= ctl->errnext;
     for (int i = 0; i < 3; ++i) ctl->smax[i] = ctl->snext[i];
   } else if (use_next == 0) {
@@ -297,6 +301,22 @@ bool chem_expansion(const evora_grid* g) {
   return g->expansion && g->floors && !g->conduction && !(g->flags & EVORA_STRICT) && !reference_backend(g);
 }
 
+// What the last physics substep of a step (the last pass over the state)
+// reduces of the next step's CFL maxima: 0 nothing (a CFL kernel follows), 1
+// in the literal, 2 in the fast forms.  chem(q) of the default mode, or the
+// gravity integration; with thermal conduction the CFL kernel also takes the
+// conduction limit.
+int physics_cfl(const evora_grid* g) {
+  if (reference_backend(g) || g->conduction || (!g->gravity && !g->floors)) return 0;
+  const bool strict = (g->flags & EVORA_STRICT) != 0;
+  if (g->floors) return !strict && (!g->expansion || chem_expansion(g)) ? 2 : 0;
+  if (g->expansion && !fused_expansion(g)) return 0;
+  return strict ? 1 : 2;
+}
+
+// Whether the CFL maxima of a step's final state are in ctl->snext after it.
+bool step_reduces_cfl(const evora_grid* g) { return g->plan.cfl_fused != 0 || physics_cfl(g) != 0; }
+
 void drop_graphs(evora_grid* g) {
   for (auto& kv : g->graphs) cudaGraphExecDestroy(kv.second);
   g->graphs.clear();
@@ -424,7 +444,7 @@ int enqueue_fused_step(evora_grid* g, bool more) {
     int rc = grav_potential(g->grav, g->qbuf[g->cur ^ 1], g->precision == EVORA_FP32, g->nf, 0, g->ctl, 1.0);
     if (!rc)
       rc = grav_integrate(g->grav, g->qbuf[g->cur ^ 1], g->precision == EVORA_FP32, g->nf, 0, g->ctl, 0.0,
-                          fused_expansion(g) ? &g->P : nullptr);
+                          &g->P, fused_expansion(g), g->floors ? 0 : physics_cfl(g));
     if (rc) return rc;
     g->launches += grav_launches(g);   // own kernels; cuFFT adds its own
   }
@@ -459,7 +479,7 @@ int enqueue_fused_step(evora_grid* g, bool more) {
   // The swap is unconditional on the host; an inactive step copies q through
   // unchanged (fused_update does that when the step is inactive).
   g->cur ^= 1;
-  g->cfl_fresh = g->plan.cfl_fused != 0;
+  g->cfl_fresh = step_reduces_cfl(g);
   return 0;
 }
 
@@ -821,7 +841,7 @@ int graph_steps(evora_grid* g, int nsteps) {
     g->launches += g->graph_launches[key];   // the kernels the capture enqueued
     if (!reference_backend(g)) {
       g->cur = start ^ (nsteps & 1);
-      g->cfl_fresh = g->plan.cfl_fused != 0;
+      g->cfl_fresh = step_reduces_cfl(g);
     }
   }
   return 0;
