@@ -27,11 +27,13 @@ Inst inst_of(int precision, int strict) {
 }
 }  // namespace
 
-// Planes per CTA of the 3D march.  The grid has tiles_xy x chunks CTAs, run
-// in waves of SMs x CTAs-per-SM; the last wave is partly empty, and every
-// chunk reloads two planes of halo.  The choice maximises
-// (waves / ceil(waves)) x zc / (zc + 2) over chunk counts with zc >= 16
-// (EVORA_ZC overrides).
+// Planes per CTA of the 3D march (EVORA_ZC overrides).  A CTA of zc planes takes
+// about zc + 5 plane times (its halo planes and the start of the pipeline), a
+// plane time 0.85 + 0.15 w with w CTAs on the SM (32^3 FP32, a CTA per SM: 3.7
+// us; 256^3, three: 4.9).  The zc with the shortest sum over the waves of
+// CTAs: few planes on small grids, whose time is one CTA's march (with at
+// least 16 planes, as this rule first had, 64^3 FP32 ran 64 CTAs for 86 us),
+// many on large ones (256^3: 52).
 int choose_zc(const HydroParams& P, int tx, int ty, int minb, int zc_default) {
   if (const char* e = getenv("EVORA_ZC")) {
     const int z = atoi(e);
@@ -41,17 +43,17 @@ int choose_zc(const HydroParams& P, int tx, int ty, int minb, int zc_default) {
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaGetLastError();
   const long long tiles_xy = (long long)((P.nx + tx - 1) / tx) * ((P.ny + ty - 1) / ty);
-  const double slots = (double)sms * (minb > 0 ? minb : 1);
-  double best = -1.0;
+  const int resident = minb > 0 ? minb : 1;
+  double best = 1e300;
   int best_zc = zc_default;
   for (int chunks = 1; chunks <= P.nz; ++chunks) {
     const int zc = (P.nz + chunks - 1) / chunks;
-    if (zc < 16 && chunks > 1) break;
     if ((P.nz + zc - 1) / zc != chunks) continue;   // the same split as a smaller count
-    const double waves = (double)(tiles_xy * chunks) / slots;
-    const double score = waves / std::ceil(waves) * (double)zc / (zc + 2);
-    if (score > best + 1e-9) {
-      best = score;
+    const long long per_sm = (tiles_xy * chunks + sms - 1) / sms;
+    const long long full = per_sm / resident, rest = per_sm % resident;
+    const double t = (zc + 5) * (full * (0.85 + 0.15 * resident) + (rest ? 0.85 + 0.15 * rest : 0.0));
+    if (t < best - 1e-9) {
+      best = t;
       best_zc = zc;
     }
   }
