@@ -28,13 +28,15 @@ Inst inst_of(int precision, int strict) {
 }  // namespace
 
 // Planes per CTA of the 3D march (EVORA_ZC overrides).  A CTA of zc planes takes
-// about zc + 5 plane times (its halo planes and the start of the pipeline), a
-// plane time 0.85 + 0.15 w with w CTAs on the SM (32^3 FP32, a CTA per SM: 3.7
-// us; 256^3, three: 4.9).  The zc with the shortest sum over the waves of
-// CTAs: few planes on small grids, whose time is one CTA's march (with at
-// least 16 planes, as this rule first had, 64^3 FP32 ran 64 CTAs for 86 us),
-// many on large ones (256^3: 52).
-int choose_zc(const HydroParams& P, int tx, int ty, int minb, int zc_default) {
+// zc + 2 plane times, a plane time going with 0.7, 0.85 and 1 for one, two and
+// three CTAs on the SM (128^3 FP32, three: 5.7 us; a CTA alone: 3.3).  Up to
+// one wave the busiest SM decides; beyond it a started wave counts between
+// its share of the SMs and a whole one (the CTAs of later waves start as
+// others end): measured over the splits of 120^3 and 128^3, 0.2 to 0.6 of the
+// way in FP32, 0.9 to 1 in FP64.  Few planes on small grids, whose time is one CTA's march
+// (with at least 16 planes, as this rule first had, 64^3 FP32 ran 64 CTAs for 86
+// us), many on large ones.
+int choose_zc(const HydroParams& P, int precision, int tx, int ty, int minb, int zc_default) {
   if (const char* e = getenv("EVORA_ZC")) {
     const int z = atoi(e);
     if (z > 0) return z;
@@ -44,14 +46,20 @@ int choose_zc(const HydroParams& P, int tx, int ty, int minb, int zc_default) {
   cudaGetLastError();
   const long long tiles_xy = (long long)((P.nx + tx - 1) / tx) * ((P.ny + ty - 1) / ty);
   const int resident = minb > 0 ? minb : 1;
+  auto share = [&](double ctas) {   // plane time with ceil(ctas) on an SM, relative to a full one
+    return 1.0 - 0.15 * (resident - std::ceil(ctas));
+  };
+  const double whole = precision == EVORA_FP32 ? 0.45 : 1.0;
   double best = 1e300;
   int best_zc = zc_default;
   for (int chunks = 1; chunks <= P.nz; ++chunks) {
     const int zc = (P.nz + chunks - 1) / chunks;
     if ((P.nz + zc - 1) / zc != chunks) continue;   // the same split as a smaller count
-    const long long per_sm = (tiles_xy * chunks + sms - 1) / sms;
-    const long long full = per_sm / resident, rest = per_sm % resident;
-    const double t = (zc + 5) * (full * (0.85 + 0.15 * resident) + (rest ? 0.85 + 0.15 * rest : 0.0));
+    const double per_sm = (double)(tiles_xy * chunks) / sms, waves = per_sm / resident;
+    const double frac = waves - std::floor(waves);
+    double t = share(per_sm);
+    if (waves > 1.0) t = waves + (frac > 0.0 ? whole * (share(frac * resident) - frac) : 0.0);
+    t *= zc + 2;
     if (t < best - 1e-9) {
       best = t;
       best_zc = zc;
@@ -94,7 +102,7 @@ void fused_set_tile(FusedPlan* pl, int tile) {
   pl->tile = tile;
   pl->launch = in.pick(pl->nf, pl->dim, tile, &pl->tx, &pl->ty, &pl->zc, &pl->smem, &pl->threads, &pl->minb);
   const HydroParams& P = pl->P;
-  if (pl->dim == 3) pl->zc = choose_zc(P, pl->tx, pl->ty, pl->minb, pl->zc);
+  if (pl->dim == 3) pl->zc = choose_zc(P, pl->precision, pl->tx, pl->ty, pl->minb, pl->zc);
   if (pl->dim == 1) {
     int64_t b = (P.nx + 127) / 128;
     pl->grid = dim3((unsigned)(b < 1 ? 1 : b), 1, 1);
