@@ -27,15 +27,26 @@ Inst inst_of(int precision, int strict) {
 }
 }  // namespace
 
-// Planes per CTA of the 3D march (EVORA_ZC overrides).  A CTA of zc planes takes
-// zc + 2 plane times, a plane time going with 0.7, 0.85 and 1 for one, two and
-// three CTAs on the SM (128^3 FP32, three: 5.7 us; a CTA alone: 3.3).  Up to
-// one wave the busiest SM decides; beyond it a started wave counts between
-// its share of the SMs and a whole one (the CTAs of later waves start as
-// others end): measured over the splits of 120^3 and 128^3, 0.2 to 0.6 of the
-// way in FP32, 0.9 to 1 in FP64.  Few planes on small grids, whose time is one CTA's march
-// (with at least 16 planes, as this rule first had, 64^3 FP32 ran 64 CTAs for 86
-// us), many on large ones.
+// The time of the 3D march in plane times of a full SM.  A CTA of zc planes
+// takes zc + 2 plane times, a plane time going with 0.7, 0.85 and 1 for one,
+// two and three CTAs on the SM (128^3 FP32, three: 5.7 us; a CTA alone: 3.3).
+// Up to one wave the busiest SM decides; beyond it a started wave counts
+// between its share of the SMs and a whole one (the CTAs of later waves start
+// as others end): measured over the splits of 120^3 and 128^3, 0.2 to 0.6 of
+// the way in FP32, 0.9 to 1 in FP64.
+double march_time(int precision, int sms, int resident, double ctas, int zc) {
+  auto share = [&](double c) { return 1.0 - 0.15 * (resident - std::ceil(c)); };
+  const double whole = precision == EVORA_FP32 ? 0.45 : 1.0;
+  const double per_sm = ctas / sms, waves = per_sm / resident, frac = waves - std::floor(waves);
+  double t = share(per_sm);
+  if (waves > 1.0) t = waves + (frac > 0.0 ? whole * (share(frac * resident) - frac) : 0.0);
+  return t * (zc + 2);
+}
+
+// Planes per CTA of the 3D march (EVORA_ZC overrides): the shortest
+// march_time.  Few planes on small grids, whose time is one CTA's march (with
+// at least 16 planes, as this rule first had, 64^3 FP32 ran 64 CTAs for 86 us),
+// many on large ones.
 int choose_zc(const HydroParams& P, int precision, int tx, int ty, int minb, int zc_default) {
   if (const char* e = getenv("EVORA_ZC")) {
     const int z = atoi(e);
@@ -45,21 +56,12 @@ int choose_zc(const HydroParams& P, int precision, int tx, int ty, int minb, int
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaGetLastError();
   const long long tiles_xy = (long long)((P.nx + tx - 1) / tx) * ((P.ny + ty - 1) / ty);
-  const int resident = minb > 0 ? minb : 1;
-  auto share = [&](double ctas) {   // plane time with ceil(ctas) on an SM, relative to a full one
-    return 1.0 - 0.15 * (resident - std::ceil(ctas));
-  };
-  const double whole = precision == EVORA_FP32 ? 0.45 : 1.0;
   double best = 1e300;
   int best_zc = zc_default;
   for (int chunks = 1; chunks <= P.nz; ++chunks) {
     const int zc = (P.nz + chunks - 1) / chunks;
     if ((P.nz + zc - 1) / zc != chunks) continue;   // the same split as a smaller count
-    const double per_sm = (double)(tiles_xy * chunks) / sms, waves = per_sm / resident;
-    const double frac = waves - std::floor(waves);
-    double t = share(per_sm);
-    if (waves > 1.0) t = waves + (frac > 0.0 ? whole * (share(frac * resident) - frac) : 0.0);
-    t *= zc + 2;
+    const double t = march_time(precision, sms, minb > 0 ? minb : 1, (double)(tiles_xy * chunks), zc);
     if (t < best - 1e-9) {
       best = t;
       best_zc = zc;
@@ -163,11 +165,9 @@ void fused_steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaS
   else f64::steps1d(pl, q, ctl, nsteps, st);
 }
 
-MultiLaunch fused_multi_pick(int precision, int strict, int nf, int* tx, int* ty, int* zc, size_t* smem,
-                             int* threads, int* ctas_per_sm) {
-  if (precision == EVORA_FP32) return f32::multi_pick(nf, tx, ty, zc, smem, threads, ctas_per_sm);
-  if (strict) return f64s::multi_pick(nf, tx, ty, zc, smem, threads, ctas_per_sm);
-  return f64::multi_pick(nf, tx, ty, zc, smem, threads, ctas_per_sm);
+MultiLaunch fused_multi_pick(int precision, int strict, int nf, MultiShape* s) {
+  if (precision == EVORA_FP32) return f32::multi_pick(nf, s);
+  return strict ? f64s::multi_pick(nf, s) : f64::multi_pick(nf, s);
 }
 
 void fused_update(const FusedPlan& pl, const void* qin, void* qout, GridCtl* ctl, cudaStream_t st) {

@@ -103,19 +103,28 @@ struct MultiGridDesc {
   int64_t n;
   int zc, dim, par, fresh;
 };
-// One work item of a batched update: a tile (bx, by, bz) of grid `grid`.
+// One work item of a batched update: a 3D tile (bx, by, bz) of grid `grid`, or
+// a 2D grid's warps of the march from warp bx on.
 struct MultiGridItem {
   int grid, bx, by, bz;
 };
-// meta[0] grids, meta[1] items, meta[2] the next item to take (reset by the
-// control kernel of each step).
-typedef void (*MultiLaunch)(const MultiGridDesc* grids, const MultiGridItem* items, int* meta, int ctas,
-                            cudaStream_t st);
+// The words of meta: grids, 3D items and the next one to take, 2D items (they
+// follow the 3D ones in the list) and the next one; the two queues are reset
+// by the control kernel of each step.
+enum { kMetaGrids = 0, kMetaItems3 = 1, kMetaNext3 = 2, kMetaItems2 = 3, kMetaNext2 = 4, kMetaWords = 8 };
+typedef void (*MultiLaunch)(const MultiGridDesc* grids, const MultiGridItem* items, int* meta, bool has3, bool has2,
+                            int sms, cudaStream_t st3, cudaStream_t st2);
 
-// The multi-grid update of a precision (tile shape, shared memory, threads
-// and CTAs per SM of its persistent launch).
-MultiLaunch fused_multi_pick(int precision, int strict, int nf, int* tx, int* ty, int* zc, size_t* smem,
-                             int* threads, int* ctas_per_sm);
+// The multi-grid update of a precision: its 3D tile and CTAs per SM, the
+// columns of a 2D warp and the warps of a 2D item.
+struct MultiShape {
+  int tx = 0, ty = 0, ctas_per_sm = 1, cols2 = 0, warps2 = 0;
+};
+MultiLaunch fused_multi_pick(int precision, int strict, int nf, MultiShape* s);
+
+// The relative time of `ctas` 3D tiles of zc planes each on sms SMs with
+// `resident` CTAs (the model the plan chooses the planes per CTA by).
+double march_time(int precision, int sms, int resident, double ctas, int zc);
 
 // Instantiation launchers (fused_f64.cu, fused_f64_strict.cu, fused_f32.cu).
 #define EVORA_DECLARE_FUSED_NS(ns)                                                           \
@@ -123,7 +132,7 @@ MultiLaunch fused_multi_pick(int precision, int strict, int nf, int* tx, int* ty
   FusedLaunch pick(int nf, int dim, int tile, int* tx, int* ty, int* zc, size_t* smem, int* threads, int* minb); \
   int tiles();                                                                               \
   bool tile_fits(const HydroParams& P, int nf, int dim, int tile);                           \
-  MultiLaunch multi_pick(int nf, int* tx, int* ty, int* zc, size_t* smem, int* threads, int* ctas_per_sm); \
+  MultiLaunch multi_pick(int nf, MultiShape* s);                                             \
   void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st);                \
   int steps1d_plan(const FusedPlan& pl);                                                     \
   void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);      \

@@ -239,10 +239,33 @@ FusedLaunch pick(int nf, int dim, int tile, int* tx, int* ty, int* zc, size_t* s
   }
 }
 
-// ---- multi-grid batches: one persistent launch updates the tiles of many
-// 2D and 3D grids of uneven sizes (the tile program of entry 0), pulling
-// (grid, tile) items from an atomic work queue; each grid keeps its own dt,
-// control block and ping-pong parity (MultiGridDesc).
+// ---- multi-grid batches: per step one persistent launch over the tiles of
+// the 3D members (the tile program of entry 0) and one over the strips of the
+// 2D members (the march), each pulling items from an atomic work queue; every
+// grid keeps its own dt, control block and ping-pong parity (MultiGridDesc).
+//
+// The two launches share no data; the batch runs them in parallel branches of
+// its graph, so that one's CTAs start as the other's run out of items.
+// 12 grids (3.6 M cells in 2D, 1.1 M in 3D), FP32: 425 -> 219 us per
+// step (one launch over tiles of both kinds, 32 planes per 3D item, before).
+template <typename Args>
+__device__ __forceinline__ void multi_args(Args& A, const MultiGridDesc& d) {
+  // the parameters by all threads, word by word
+  static_assert(sizeof(HydroParams) % 4 == 0, "copied by words");
+  const unsigned* src = reinterpret_cast<const unsigned*>(&d.P);
+  unsigned* dst = reinterpret_cast<unsigned*>(&A.P);
+  for (int i = threadIdx.x; i < (int)(sizeof(HydroParams) / 4); i += blockDim.x) dst[i] = src[i];
+  if (threadIdx.x == 0) {
+    A.qin = (const TT*)d.q[d.par];
+    A.qout = (TT*)d.q[d.par ^ 1];
+    A.ctl = d.ctl;
+    A.n = d.n;
+    A.cfl_next = 1;
+    A.zc = d.zc;
+    A.tail = 0;
+  }
+}
+
 template <int NF>
 __global__ void __launch_bounds__(Tile<0>::TX* Tile<0>::TY, Tile<0>::MINB)
     k_multi(const MultiGridDesc* grids, const MultiGridItem* items, int* meta) {
@@ -250,58 +273,73 @@ __global__ void __launch_bounds__(Tile<0>::TX* Tile<0>::TY, Tile<0>::MINB)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& sm = *reinterpret_cast<FusedSmem<TT, NF, C::TX, C::TY>*>(smem_raw);
   __shared__ __align__(16) unsigned char a_raw[sizeof(FusedArgs<TT>)];
-  __shared__ int s_item, s_dim, s_bx, s_by, s_bz;
+  __shared__ int s_item;
   auto& A = *reinterpret_cast<FusedArgs<TT>*>(a_raw);
-  const int nitems = meta[1];
+  const int nitems = meta[kMetaItems3];
   for (;;) {
-    if (threadIdx.x == 0) {
-      const int it = atomicAdd(&meta[2], 1);
-      s_item = it;
-      if (it < nitems) {
-        const MultiGridItem w = items[it];
-        const MultiGridDesc& d = grids[w.grid];
-        A.P = d.P;
-        A.qin = (const TT*)d.q[d.par];
-        A.qout = (TT*)d.q[d.par ^ 1];
-        A.ctl = d.ctl;
-        A.n = d.n;
-        A.cfl_next = 1;
-        A.zc = d.zc;
-        s_dim = d.dim;
-        s_bx = w.bx;
-        s_by = w.by;
-        s_bz = w.bz;
-      }
-    }
+    if (threadIdx.x == 0) s_item = atomicAdd(&meta[kMetaNext3], 1);
     __syncthreads();
     if (s_item >= nitems) break;
-    if (s_dim == 3) fused_tile<TT, NF, 3, C::TX, C::TY, C::ZC>(A, sm, threadIdx.x, s_bx, s_by, s_bz);
-    else fused_tile<TT, NF, 2, C::TX, C::TY, C::ZC>(A, sm, threadIdx.x, s_bx, s_by, 0);
+    const MultiGridItem w = items[s_item];
+    multi_args(A, grids[w.grid]);
+    __syncthreads();
+    fused_tile<TT, NF, 3, C::TX, C::TY, C::ZC>(A, sm, threadIdx.x, w.bx, w.by, w.bz);
+    __syncthreads();   // the shared state is reused by the next item
+  }
+}
+
+// A 2D item: kMarchWarps warps of the march from warp bx on.
+template <int NF>
+__global__ void __launch_bounds__(32 * kMarchWarps, sizeof(TT) == 4 ? 4 : 3)
+    k_multi2d(const MultiGridDesc* grids, const MultiGridItem* items, int* meta) {
+  __shared__ __align__(16) unsigned char a_raw[sizeof(FusedArgs<TT>)];
+  __shared__ TT red[3][kMarchWarps];
+  __shared__ int s_item;
+  auto& A = *reinterpret_cast<FusedArgs<TT>*>(a_raw);
+  const int nitems = meta[kMetaItems2];
+  items += meta[kMetaItems3];
+  for (;;) {
+    if (threadIdx.x == 0) s_item = atomicAdd(&meta[kMetaNext2], 1);
+    __syncthreads();
+    if (s_item >= nitems) break;
+    const MultiGridItem w = items[s_item];
+    multi_args(A, grids[w.grid]);
+    __syncthreads();
+    TT cm[3] = {(TT)0, (TT)0, (TT)0};
+    unsigned cerr = 0;
+    const int gw = w.bx + (int)(threadIdx.x >> 5);
+    if (A.P.limiter == 1 && A.P.solver == 2 && A.P.secondorder) march2d<TT, NF, true>(A, gw, cm, cerr);
+    else march2d<TT, NF, false>(A, gw, cm, cerr);
+    march_maxima(A.ctl, cm, cerr, red);
     __syncthreads();   // the shared state is reused by the next item
   }
 }
 
 template <int NF>
-void multi_launch(const MultiGridDesc* grids, const MultiGridItem* items, int* meta, int ctas, cudaStream_t st) {
+void multi_launch(const MultiGridDesc* grids, const MultiGridItem* items, int* meta, bool has3, bool has2, int sms,
+                  cudaStream_t st3, cudaStream_t st2) {
   using C = Tile<0>;
-  k_multi<NF><<<ctas, C::TX * C::TY, sizeof(FusedSmem<TT, NF, C::TX, C::TY>), st>>>(grids, items, meta);
+  if (has3)
+    k_multi<NF><<<sms * C::MINB, C::TX * C::TY, sizeof(FusedSmem<TT, NF, C::TX, C::TY>), st3>>>(grids, items, meta);
+  if (has2)
+    k_multi2d<NF><<<sms * (sizeof(TT) == 4 ? 4 : 3), 32 * kMarchWarps, 0, st2>>>(grids, items, meta);
 }
 
-MultiLaunch multi_pick(int nf, int* tx, int* ty, int* zc, size_t* smem, int* threads, int* ctas_per_sm) {
+MultiLaunch multi_pick(int nf, MultiShape* s) {
   using C = Tile<0>;
-  *tx = C::TX;
-  *ty = C::TY;
-  *zc = C::ZC;
-  *threads = C::TX * C::TY;
-  *ctas_per_sm = C::MINB;
+  s->tx = C::TX;
+  s->ty = C::TY;
+  s->ctas_per_sm = C::MINB;
+  s->cols2 = kMarchCols;
+  s->warps2 = kMarchWarps;
   if (nf == 5) {
-    *smem = sizeof(FusedSmem<TT, 5, C::TX, C::TY>);
-    cudaFuncSetAttribute(k_multi<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
+    cudaFuncSetAttribute(k_multi<5>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sizeof(FusedSmem<TT, 5, C::TX, C::TY>));
     cudaFuncSetAttribute(k_multi<5>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return &multi_launch<5>;
   }
-  *smem = sizeof(FusedSmem<TT, 6, C::TX, C::TY>);
-  cudaFuncSetAttribute(k_multi<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
+  cudaFuncSetAttribute(k_multi<6>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(FusedSmem<TT, 6, C::TX, C::TY>));
   cudaFuncSetAttribute(k_multi<6>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   return &multi_launch<6>;
 }

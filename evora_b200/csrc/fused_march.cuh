@@ -161,6 +161,25 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
   if (err) atomicOr(&A.ctl->err, err);
 }
 
+// A CTA's maxima and errors into its grid's control block (all threads).
+template <typename T>
+__device__ __forceinline__ void march_maxima(GridCtl* ctl, const T* cm, unsigned cerr, T (*red)[kMarchWarps]) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const T m = warp_max_pos(cm[d]);
+    if (lane == 0) red[d][wid] = m;
+  }
+  if (cerr) atomicOr(&ctl->errnext, cerr);
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    T m = red[threadIdx.x][0];
+#pragma unroll
+    for (int k = 1; k < kMarchWarps; ++k) m = fmax2(m, red[threadIdx.x][k]);
+    atomicMax(&ctl->snext[threadIdx.x], ordered_bits((double)m));
+  }
+}
+
 // OPT: grids with the usual options (minmod, HLLC, second order), as
 // constants (1024^2 FP32: 43 -> 33 us).  CTAs per SM: FP32 needs 115 registers,
 // so 4; FP64 at 3 (168 registers) or 4 (128, with spills) takes 27 or 30 us at
@@ -168,26 +187,11 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
 template <typename T, int NF, bool OPT>
 __global__ void __launch_bounds__(32 * kMarchWarps, sizeof(T) == 4 ? 4 : 3) k_march2d(FusedArgs<T> A) {
   __shared__ T red[3][kMarchWarps];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   T cm[3] = {(T)0, (T)0, (T)0};
   unsigned cerr = 0;
   step_head();
-  march2d<T, NF, OPT>(A, blockIdx.x * kMarchWarps + wid, cm, cerr);
-  if (A.cfl_next) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const T m = warp_max_pos(cm[d]);
-      if (lane == 0) red[d][wid] = m;
-    }
-    if (cerr) atomicOr(&A.ctl->errnext, cerr);
-    __syncthreads();
-    if (threadIdx.x < 3) {
-      T m = red[threadIdx.x][0];
-#pragma unroll
-      for (int k = 1; k < kMarchWarps; ++k) m = fmax2(m, red[threadIdx.x][k]);
-      atomicMax(&A.ctl->snext[threadIdx.x], ordered_bits((double)m));
-    }
-  }
+  march2d<T, NF, OPT>(A, blockIdx.x * kMarchWarps + (threadIdx.x >> 5), cm, cerr);
+  if (A.cfl_next) march_maxima(A.ctl, cm, cerr, red);
   step_tail(A);
 }
 

@@ -99,17 +99,20 @@ struct evora_multigrid {
   int nf = 5;
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaStream_t side = nullptr;             // the 2D members' branch of a step
+  cudaEvent_t forked = nullptr, joined = nullptr;
   std::vector<evora_grid*> grids;
   bool dirty = true;
   evora::MultiGridDesc* d_desc = nullptr;
   evora::MultiGridItem* d_items = nullptr;
-  int* d_meta = nullptr;                   // grids, items, next item
+  int* d_meta = nullptr;                   // kMeta* words
   long long* d_status = nullptr;           // per grid: go | err << 1, then k
   int cap_grids = 0, cap_items = 0;
   evora::MultiLaunch launch = nullptr;
-  int tx = 0, ty = 0, zc = 0, threads = 0, ctas = 0;
-  size_t smem = 0;
-  std::map<int, cudaGraphExec_t> graphs;   // by step count
+  evora::MultiShape shape;
+  int sms = 148;
+  bool has3 = false, has2 = false;         // the kinds of members
+  std::map<int, cudaGraphExec_t> graphs;   // by step count and kinds of members
   long long cell_updates = 0;              // member cells x steps enqueued
 };
 
@@ -228,27 +231,26 @@ __global__ void k_step_control(HydroParams P, GridCtl* ctl, int end) {
   step_time(P, ctl);
 }
 
-// Control of a multi-grid step, one thread per grid: hydrostep part 2 and
-// updatetime (as k_step_begin + k_step_time), and after the update the step
-// count, the ping-pong parity and a compact status word.
-__global__ void k_mg_begin(MultiGridDesc* g, int* meta) {
+// Control between the updates of a multi-grid batch, one thread per grid.
+// end: after an update, the step count, the ping-pong parity and a compact
+// status word; begin: before one, hydrostep part 2 and updatetime (as
+// k_step_begin + k_step_time).
+__global__ void k_mg_control(MultiGridDesc* g, int* meta, long long* status, int end, int begin) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) meta[2] = 0;
-  if (i >= meta[0]) return;
+  if (i == 0) meta[kMetaNext3] = meta[kMetaNext2] = 0;
+  if (i >= meta[kMetaGrids]) return;
   GridCtl* ctl = g[i].ctl;
-  step_begin(ctl, g[i].fresh ? 1 : 2);
-  g[i].fresh = 1;
-  step_time(g[i].P, ctl);
-}
-
-__global__ void k_mg_end(MultiGridDesc* g, const int* meta, long long* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= meta[0]) return;
-  GridCtl* ctl = g[i].ctl;
-  step_end(ctl);
-  g[i].par ^= 1;
-  status[2 * i] = (long long)(ctl->go != 0) | ((long long)ctl->err << 1);
-  status[2 * i + 1] = ctl->k;
+  if (end) {
+    step_end(ctl);
+    g[i].par ^= 1;
+    status[2 * i] = (long long)(ctl->go != 0) | ((long long)ctl->err << 1);
+    status[2 * i + 1] = ctl->k;
+  }
+  if (begin) {
+    step_begin(ctl, g[i].fresh ? 1 : 2);
+    g[i].fresh = 1;
+    step_time(g[i].P, ctl);
+  }
 }
 
 // An update with the caller's dt (the drop-in layer's resident mode): the
@@ -1111,6 +1113,35 @@ int mg_rebuild(evora_multigrid* m) {
     const evora_grid* gb = m->grids[b];
     return (int64_t)ga->P.nx * ga->P.ny * ga->P.nz > (int64_t)gb->P.nx * gb->P.ny * gb->P.nz;
   });
+  // one number of planes per 3D tile and of rows per 2D warp for all members:
+  // the planes with the shortest time of all their tiles, rows that give the
+  // 2D queue about two rounds of warps
+  const MultiShape& sh = m->shape;
+  int zmax = 0, zc = 1;
+  double rows = 0.0, best = 1e300;
+  m->has3 = m->has2 = false;
+  for (const evora_grid* g : m->grids) {
+    if (g->plan.dim == 3) {
+      zmax = std::max(zmax, g->P.nz);
+      m->has3 = true;
+    } else {
+      rows += (double)((g->P.nx + sh.cols2 - 1) / sh.cols2) * g->P.ny;
+      m->has2 = true;
+    }
+  }
+  for (int z = 2; z <= std::min(zmax, 64); ++z) {
+    double ctas = 0.0;
+    for (const evora_grid* g : m->grids)
+      if (g->plan.dim == 3)
+        ctas += (double)((g->P.nx + sh.tx - 1) / sh.tx) * ((g->P.ny + sh.ty - 1) / sh.ty) * ((g->P.nz + z - 1) / z);
+    const double t = march_time(m->precision, m->sms, sh.ctas_per_sm, ctas, z);
+    if (t < best) {
+      best = t;
+      zc = z;
+    }
+  }
+  const double resident = (double)m->sms * (m->precision == EVORA_FP32 ? 16 : 12);
+  const int r2 = std::max(2, std::min(16, (int)(rows / (2.0 * resident) + 0.999)));
   for (int i = 0; i < n; ++i) {
     evora_grid* g = m->grids[i];
     MultiGridDesc& d = desc[i];
@@ -1120,20 +1151,24 @@ int mg_rebuild(evora_multigrid* m) {
     d.ctl = g->ctl;
     d.n = ncells(g);
     d.dim = g->plan.dim;
-    d.zc = d.dim == 3 ? std::min(m->zc, g->P.nz) : 1;
+    d.zc = d.dim == 3 ? zc : r2;
     d.par = g->cur;
     d.fresh = g->cfl_fresh ? 1 : 0;
   }
   for (int i : idx) {
     const MultiGridDesc& d = desc[i];
-    const int gx = (d.P.nx + m->tx - 1) / m->tx, gy = (d.P.ny + m->ty - 1) / m->ty;
-    const int gz = d.dim == 3 ? (d.P.nz + d.zc - 1) / d.zc : 1;
-    auto& dst = d.dim == 3 ? items3 : items2;
-    for (int bz = 0; bz < gz; ++bz)
-      for (int by = 0; by < gy; ++by)
-        for (int bx = 0; bx < gx; ++bx) dst.push_back(MultiGridItem{i, bx, by, bz});
+    if (d.dim == 3) {
+      const int gx = (d.P.nx + sh.tx - 1) / sh.tx, gy = (d.P.ny + sh.ty - 1) / sh.ty, gz = (d.P.nz + zc - 1) / zc;
+      for (int bz = 0; bz < gz; ++bz)
+        for (int by = 0; by < gy; ++by)
+          for (int bx = 0; bx < gx; ++bx) items3.push_back(MultiGridItem{i, bx, by, bz});
+    } else {
+      const int warps = ((d.P.nx + sh.cols2 - 1) / sh.cols2) * ((d.P.ny + r2 - 1) / r2);
+      for (int w = 0; w < warps; w += sh.warps2) items2.push_back(MultiGridItem{i, w, 0, 0});
+    }
   }
-  items3.insert(items3.end(), items2.begin(), items2.end());   // 3D items (ZC planes) before 2D ones
+  const int n3 = (int)items3.size(), n2 = (int)items2.size();
+  items3.insert(items3.end(), items2.begin(), items2.end());
   const int ni = (int)items3.size();
   if (n > m->cap_grids || ni > m->cap_items) {
     CU(cudaStreamSynchronize(m->stream));
@@ -1157,7 +1192,7 @@ int mg_rebuild(evora_multigrid* m) {
       m->cap_items = cap;
     }
   }
-  const int meta[3] = {n, ni, 0};
+  const int meta[kMetaWords] = {n, n3, 0, n2, 0};
   if (n) CU(cudaMemcpyAsync(m->d_desc, desc.data(), sizeof(MultiGridDesc) * n, cudaMemcpyHostToDevice, m->stream));
   if (ni) CU(cudaMemcpyAsync(m->d_items, items3.data(), sizeof(MultiGridItem) * ni, cudaMemcpyHostToDevice, m->stream));
   CU(cudaMemcpyAsync(m->d_meta, meta, sizeof meta, cudaMemcpyHostToDevice, m->stream));
@@ -1177,10 +1212,20 @@ int mg_rebuild(evora_multigrid* m) {
 void mg_enqueue(evora_multigrid* m, int nsteps) {
   const int cb = (m->cap_grids + 127) / 128;
   for (int k = 0; k < nsteps; ++k) {
-    k_mg_begin<<<cb, 128, 0, m->stream>>>(m->d_desc, m->d_meta);
-    m->launch(m->d_desc, m->d_items, m->d_meta, m->ctas, m->stream);
-    k_mg_end<<<cb, 128, 0, m->stream>>>(m->d_desc, m->d_meta, m->d_status);
+    k_mg_control<<<cb, 128, 0, m->stream>>>(m->d_desc, m->d_meta, m->d_status, k > 0, 1);
+    // 2D and 3D members side by side (in a captured graph: parallel branches)
+    const bool fork = m->stream && m->has3 && m->has2;
+    if (fork) {
+      cudaEventRecord(m->forked, m->stream);
+      cudaStreamWaitEvent(m->side, m->forked, 0);
+    }
+    m->launch(m->d_desc, m->d_items, m->d_meta, m->has3, m->has2, m->sms, m->stream, fork ? m->side : m->stream);
+    if (fork) {
+      cudaEventRecord(m->joined, m->side);
+      cudaStreamWaitEvent(m->stream, m->joined, 0);
+    }
   }
+  k_mg_control<<<cb, 128, 0, m->stream>>>(m->d_desc, m->d_meta, m->d_status, 1, 0);
 }
 
 bool mg_accepts(const evora_multigrid* m, const evora_grid* g) {
@@ -1205,14 +1250,14 @@ int evora_multigrid_create(int32_t precision, int32_t flags, void* stream, evora
   m->nf = (flags & EVORA_CARRY_ENTROPY) ? 6 : 5;
   m->stream = (cudaStream_t)stream;
   cudaGetDevice(&m->device);
-  int per_sm = 1, sms = 148;
-  m->launch = fused_multi_pick(precision, (flags & EVORA_STRICT) != 0, m->nf, &m->tx, &m->ty, &m->zc, &m->smem,
-                               &m->threads, &per_sm);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-  m->ctas = sms * per_sm;
-  if (cudaMalloc(&m->d_meta, sizeof(int) * 4) != cudaSuccess) {
+  m->launch = fused_multi_pick(precision, (flags & EVORA_STRICT) != 0, m->nf, &m->shape);
+  cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
+  if (cudaMalloc(&m->d_meta, sizeof(int) * kMetaWords) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->forked, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->joined, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
-    delete m;
+    evora_multigrid_destroy(m);
     return EVORA_ERR_NOMEM;
   }
   *out = m;
@@ -1228,6 +1273,9 @@ int evora_multigrid_destroy(evora_multigrid* m) {
   cudaFree(m->d_items);
   cudaFree(m->d_meta);
   cudaFree(m->d_status);
+  if (m->forked) cudaEventDestroy(m->forked);
+  if (m->joined) cudaEventDestroy(m->joined);
+  if (m->side) cudaStreamDestroy(m->side);
   delete m;
   return 0;
 }
@@ -1266,7 +1314,8 @@ int evora_multigrid_step(evora_multigrid* m, int32_t nsteps, int32_t sync) {
   while (left > 0) {
     const int chunk = left < 32 ? left : 32;
     if (m->stream) {
-      auto it = m->graphs.find(chunk);
+      const int key = 4 * chunk + 2 * m->has3 + m->has2;
+      auto it = m->graphs.find(key);
       if (it == m->graphs.end()) {
         cudaGraph_t graph;
         CU(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
@@ -1283,7 +1332,7 @@ int evora_multigrid_step(evora_multigrid* m, int32_t nsteps, int32_t sync) {
           set_cuda_error(e, "evora_multigrid_step: instantiate");
           return EVORA_ERR_CUDA;
         }
-        it = m->graphs.emplace(chunk, exec).first;
+        it = m->graphs.emplace(key, exec).first;
       }
       CU(cudaGraphLaunch(it->second, m->stream));
     } else {
@@ -1295,7 +1344,7 @@ int evora_multigrid_step(evora_multigrid* m, int32_t nsteps, int32_t sync) {
   for (evora_grid* g : m->grids) {
     if (nsteps & 1) g->cur ^= 1;
     g->cfl_fresh = g->plan.cfl_fused != 0;
-    g->launches += 3LL * nsteps;
+    g->launches += (1LL + m->has3 + m->has2) * nsteps + 1;
     m->cell_updates += (long long)nsteps * ncells(g);
   }
   if (sync) CU(cudaStreamSynchronize(m->stream));

@@ -91,3 +91,49 @@ def test_tail_control_ends_and_stops(cuda_device, dims):
     assert g.status() & 1 and g.time()["k"] == 0
     np.testing.assert_array_equal(g.get_q()[..., :5], bad[..., :5])
     g.close()
+
+
+@pytest.mark.parametrize("precision,flags", [(ev.FP64, ev.STRICT), (ev.FP32, 0)])
+def test_multigrid_kinds_of_members(cuda_device, precision, flags):
+    """Batches of 2D members, of 3D members and of both, changed between steps:
+    every member equals the grid stepped alone (strict FP64 bit for bit, FP32
+    to rounding)."""
+    import torch
+    stream = torch.cuda.Stream()
+    dims = [(57, 33, 1), (300, 70, 1), (24, 20, 18), (2, 2, 1), (33, 9, 40)]
+    kws = [dict(nx=a, ny=b, nz=c, g=5.0 / 3.0, cfl=0.4, tend=1e9, boundtype=1 + i % 3, limiter=1 + i % 2,
+                solver=2 - i % 2) for i, (a, b, c) in enumerate(dims)]
+    qs = [state(kw, i) for i, kw in enumerate(kws)]
+    grids = [ev.Grid(ev.default_params(**kw), precision, flags, stream=stream) for kw in kws]
+    for g, q in zip(grids, qs):
+        g.set_q(q)
+    mg = ev.MultiGrid(precision, flags, stream=stream)
+    steps = [0] * len(dims)
+
+    def advance(n):
+        mg.step(n)
+        for i, g in enumerate(grids):
+            if g in mg.members:
+                steps[i] += n
+    for i in (0, 1):
+        mg.add(grids[i])
+    advance(3)
+    for i in (2, 3, 4):
+        mg.add(grids[i])
+    advance(2)
+    for i in (0, 1, 3):
+        mg.remove(grids[i])
+    advance(3)
+    status = mg.status()
+    assert [k for _, _, k in status] == [steps[2], steps[4]] and all(e == 0 for _, e, _ in status)
+    mg.close()
+    for i, (kw, q) in enumerate(zip(kws, qs)):
+        with ev.Grid(ev.default_params(**kw), precision, flags) as g:
+            g.set_q(q)
+            g.step(steps[i])
+            if flags:
+                np.testing.assert_array_equal(grids[i].get_q(), g.get_q())
+            else:
+                fields = [0, 1, 2, 4]
+                assert np.all(rel_l1(grids[i].get_q(), g.get_q())[fields] <= 1e-5)
+        grids[i].close()
