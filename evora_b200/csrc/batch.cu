@@ -47,6 +47,8 @@ struct evora_batch {
   BatchLaunch launch = nullptr;
   std::map<int, cudaGraphExec_t> graphs;
   bool order_dirty = true;
+  bool clusters = true;    // the default shape: a cluster per tube where that pays (batch_cluster_for)
+  int sms = 148;
 };
 
 namespace {
@@ -223,6 +225,12 @@ int evora::batch_ctas_per_sm(int precision, int strict, int nf, int threads, siz
   return strict ? f64s::batch_max_ctas_per_sm(nf, threads, smem) : f64::batch_max_ctas_per_sm(nf, threads, smem);
 }
 
+bool evora::batch_cluster_for(int precision, int strict, const BatchPlan& pl, void* q, int running, int nmax, int sms,
+                              cudaStream_t st) {
+  if (precision == EVORA_FP32) return f32::batch_cluster(pl, q, running, nmax, sms, st);
+  return strict ? f64s::batch_cluster(pl, q, running, nmax, sms, st) : f64::batch_cluster(pl, q, running, nmax, sms, st);
+}
+
 namespace {
 
 // Range of tubes [t0, t1) and its cells for tube index `tube` (-1 = all).
@@ -321,6 +329,11 @@ int evora_batch_create(const evora_params* p, int32_t ntubes, const int32_t* n, 
   }
   b->ntot = ntot;
   b->nmax = nmax;
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaGetLastError();
+  }
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) goto fail;
   b->own_stream = true;
   if (cudaMalloc(&b->q, (size_t)b->nf * ntot * esize(b)) != cudaSuccess) goto fail;
@@ -465,7 +478,8 @@ int evora_batch_run(evora_batch* b, int32_t max_steps, int32_t sync) {
     cudaGraph_t g;
     CU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
-    b->launch(b->plan, b->q, b->stream);
+    if (!b->clusters || !batch_cluster_for(b->precision, b->strict, b->plan, b->q, b->ntubes, b->nmax, b->sms, b->stream))
+      b->launch(b->plan, b->q, b->stream);
     CU(cudaStreamEndCapture(b->stream, &g));
     cudaGraphExec_t ex;
     cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
@@ -514,6 +528,7 @@ int evora_batch_configure(evora_batch* b, int32_t threads, int32_t ctas_per_sm) 
   if (!b || (threads != 128 && threads != 256 && threads != 512) || ctas_per_sm < 1 || ctas_per_sm > 8)
     return EVORA_ERR_ARG;
   CU(cudaStreamSynchronize(b->stream));
+  b->clusters = false;
   return configure(b, threads, cap_for(b, ctas_per_sm));
 }
 
@@ -574,6 +589,7 @@ int evora_batch_autotune(evora_batch* b, int32_t steps, int32_t* threads_out, in
   cudaEventDestroy(e1);
   cudaFree(save_q);
   cudaFree(save_t);
+  b->clusters = false;
   if (threads_out) *threads_out = bt;
   if (ctas_out) *ctas_out = bc;
   return configure(b, bt, cap_for(b, bc));

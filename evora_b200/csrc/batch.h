@@ -70,6 +70,8 @@ struct BatchPlan {
   /* configures launch for nf fields and `threads` per CTA; sets plan->smem from cap */     \
   BatchLaunch batch_pick(int nf, int threads, BatchPlan* plan);                             \
   int batch_max_ctas_per_sm(int nf, int threads, size_t smem);                              \
+  /* launches a cluster of CTAs per tube where that serves `running` tubes, else false */   \
+  bool batch_cluster(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st);  \
   }
 EVORA_DECLARE_BATCH_NS(f64)
 EVORA_DECLARE_BATCH_NS(f64s)
@@ -84,5 +86,7 @@ void tube_to_aos(const void* q, double* aos, bool f32, long long ntot, long long
 // Instantiation dispatch by precision.
 BatchLaunch batch_pick_for(int precision, int strict, int nf, int threads, BatchPlan* pl);
 int batch_ctas_per_sm(int precision, int strict, int nf, int threads, size_t smem);
+bool batch_cluster_for(int precision, int strict, const BatchPlan& pl, void* q, int running, int nmax, int sms,
+                       cudaStream_t st);
 
 }  // namespace evora

@@ -151,17 +151,12 @@ __device__ __forceinline__ void tube_sweep(T* qs, const T* w, int n, const Hydro
     tube_sweep_opt<T, NF, NT>(qs, w, n, P, P.limiter, P.solver, P.secondorder != 0, c, de, dt, err);
 }
 
-template <typename T, int NF, int NT>
-__device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int tb, T* red,
-                                         unsigned* s_err) {
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  TubeState* ts = A.tubes + tb;
-  const int n = ts->n;
-  const long long off = ts->offset;
-  const HydroParams& PP = A.P;
-  // compparameter for this tube (parameter.f90:192-205, 1D branch)
-  HydroParams P = PP;
-  if (ts->bt) P.boundtype = ts->bt;
+// compparameter for a tube of n cells (parameter.f90:192-205, 1D branch);
+// bt: its boundary type (0: the batch's).
+template <typename T>
+__device__ __forceinline__ HydroParams tube_params(const BatchArgs<T>& A, int n, int bt) {
+  HydroParams P = A.P;
+  if (bt) P.boundtype = bt;
   P.nx = n;
   P.ny = 1;
   P.nz = 1;
@@ -176,6 +171,42 @@ __device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int
   P.dxinv = 1.0 / P.dx;
   P.dyinv = 1.0 / P.dy;
   P.dzinv = 1.0 / P.dz;
+  return P;
+}
+
+// The most steps a tube of n cells runs in this launch.
+template <typename T>
+__device__ __forceinline__ int tube_budget(const BatchArgs<T>& A, int n) {
+  int budget = A.budget;
+  if (A.quantum > 0) {
+    const long long b = A.quantum / n;
+    budget = (int)(b < 1 ? 1 : (b < budget ? b : budget));
+  }
+  if (A.steps_per_cell > 0.0) budget = max(1, (int)(A.steps_per_cell * n));
+  return budget;
+}
+
+// A tube's bookkeeping after a launch (one thread).
+template <typename T>
+__device__ __forceinline__ void tube_close(const BatchArgs<T>& A, TubeState* ts, int n, double t, double dt, int steps,
+                                           unsigned err, int go) {
+  ts->err |= err;
+  ts->t = t;
+  ts->dt = dt;
+  ts->k += steps;
+  if (err) ts->status = TUBE_ERROR;
+  else if (!go) ts->status = TUBE_DONE;
+  atomicAdd((unsigned long long*)A.cell_updates, (unsigned long long)n * (unsigned long long)steps);
+}
+
+template <typename T, int NF, int NT>
+__device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int tb, T* red,
+                                         unsigned* s_err) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  TubeState* ts = A.tubes + tb;
+  const int n = ts->n;
+  const long long off = ts->offset;
+  const HydroParams P = tube_params(A, n, ts->bt);
   const Gas<T> c = Gas<T>::make(P);
   const bool de = P.dualenergy != 0;
   // stage q into qs (field-major, stride n)
@@ -185,12 +216,7 @@ __device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int
   unsigned err = 0;
   int steps = 0, go = 1;
   if (tid == 0) *s_err = 0u;
-  int budget = A.budget;
-  if (A.quantum > 0) {
-    const long long b = A.quantum / n;
-    budget = (int)(b < 1 ? 1 : (b < budget ? b : budget));
-  }
-  if (A.steps_per_cell > 0.0) budget = max(1, (int)(A.steps_per_cell * n));
+  const int budget = tube_budget(A, n);
   __syncthreads();
   while (steps < budget) {
     // ---- phase 1: primitives (+ ghosts) and the CFL maximum
@@ -222,16 +248,7 @@ __device__ __forceinline__ void tube_run(const BatchArgs<T>& A, T* qs, T* w, int
   for (int f = 0; f < NF; ++f)
     for (int i = tid; i < n; i += NT) A.q[(size_t)f * A.ntot + off + i] = qs[f * n + i];
   __syncthreads();
-  if (tid == 0) {
-    const unsigned e = *s_err;
-    ts->err |= e;
-    ts->t = t;
-    ts->dt = dt;
-    ts->k += steps;
-    if (e) ts->status = TUBE_ERROR;
-    else if (!go) ts->status = TUBE_DONE;
-    atomicAdd((unsigned long long*)A.cell_updates, (unsigned long long)n * (unsigned long long)steps);
-  }
+  if (tid == 0) tube_close(A, ts, n, t, dt, steps, *s_err, go);
 }
 
 template <typename T, int NF, int NT>
@@ -269,69 +286,76 @@ __global__ void __launch_bounds__(NT) k_tubes(BatchArgs<T> A) {
   }
 }
 
-// ---- resident 1D grids: nsteps steps in one launch by one thread-block
-// cluster (the loop main.f90:109-155 with the control block's scalars).
+// ---- lines of cells shared by the CTAs of a thread-block cluster: several
+// steps of a resident 1D grid in one launch, and tubes of batches too small
+// to give every SM one (the loop main.f90:109-155).
 //
 // Rank r of the cluster keeps the cells [r m, r m + its cells) in shared
-// memory over the whole launch.  Per step it forms the primitives of its
-// cells, stores the two at either end into its neighbours' halos (or, at the
-// ends of the grid, mirrors them into its own) and its warps' maxima and
-// errors into every rank, all through distributed shared memory; one cluster
-// barrier; dt from all maxima; the sweep; one block barrier.  Halos, maxima
-// and errors are double-buffered by the step's parity: a rank that is one
-// barrier ahead writes the other copy.
-// Bound: the latency of the step's dependent chain; a step of separate kernels
-// cost 10 us however small the grid.  1024 FP64 cells: 9.0 -> 2.2 us per step;
-// by size and number of ranks: steps1d_plan (fused_inst.cuh).
+// memory over the steps.  Per step it forms the primitives of its cells,
+// stores the two at either end into its neighbours' halos (or, at the ends of
+// the line, mirrors them into its own) and its warps' maxima and errors into
+// every rank, all through distributed shared memory; one cluster barrier; dt
+// from all maxima; the sweep; one block barrier.  Halos, maxima and errors are
+// double-buffered by the step's parity: a rank that is one barrier ahead
+// writes the other copy.
+// Bound: the latency of the step's dependent chain.  Resident grid, 1024 FP64
+// cells: 9.0 (five launches per step) -> 2.2 us per step; by size and number of
+// ranks: steps1d_plan (fused_inst.cuh).
 template <typename T, int NT>
 struct LineMax {
   T smax[2][16 * (NT / 32)];
   unsigned err[2][16 * (NT / 32)];
 };
 
-template <typename T, int NF, int NT>
-__global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q, GridCtl* ctl, int nsteps, int m) {
+// The line and its running time; every thread of the cluster holds the same.
+struct LineRun {
+  double t, dt, tend;
+  int go;        // updatetime's flag
+  int active;    // the last step asked for was run (or ended in an error of its update)
+  int k;         // steps done
+  unsigned err;
+};
+
+// Up to nsteps steps of the line of n cells at q (field stride fs) by the
+// first ranks of the cluster, m cells each; the other ranks only keep step.
+// TUBE: a step whose update fails counts, and one that does not advance t
+// raises EVORA_ERR_DT (tube_run); else the control block's rules
+// (step_begin, step_time, step_end).  smem: steps1d_smem(NF, m) bytes.
+template <typename T, int NF, int NT, bool TUBE>
+__device__ __forceinline__ void line_steps(const HydroParams& P, const Gas<T>& c, bool de, T* q, int64_t fs, int n,
+                                           int m, int nsteps, bool runnable, unsigned char* smem, LineMax<T, NT>& mx,
+                                           LineRun& L) {
   namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) unsigned char sraw[];
-  __shared__ LineMax<T, NT> mx;
-  __shared__ unsigned s_err;
   constexpr int NW = NT / 32;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), nr = (int)cl.num_blocks();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int n = P.nx;
+  const int used = (n + m - 1) / m;              // ranks that have cells (each >= 2)
   const int x0 = rank * m;
-  const int mine = n - x0 < m ? n - x0 : m;      // >= 2 (the launch sees to it)
+  const int mine = rank < used ? (n - x0 < m ? n - x0 : m) : 0;
   const int wlen = 5 * (m + 4);                  // one copy of the primitives
-  T* const w0 = reinterpret_cast<T*>(sraw);
+  T* const w0 = reinterpret_cast<T*>(smem);
   T* const qs = w0 + 2 * wlen;                   // field-major, stride mine
   const int wst = mine + 4;
   // the neighbours' primitives and row strides
   const bool periodic = P.boundtype == 2;
-  const int lr = rank > 0 ? rank - 1 : (periodic ? nr - 1 : -1);
-  const int ur = rank < nr - 1 ? rank + 1 : (periodic ? 0 : -1);
+  const int lr = rank > 0 ? rank - 1 : (periodic ? used - 1 : -1);
+  const int ur = rank < used - 1 ? rank + 1 : (periodic ? 0 : -1);
   auto cells_of = [&](int r) { return n - r * m < m ? n - r * m : m; };
   T* const wl = lr >= 0 ? cl.map_shared_rank(w0, lr) : w0;
   T* const wu = ur >= 0 ? cl.map_shared_rank(w0, ur) : w0;
   const int ml = lr >= 0 ? cells_of(lr) : mine, mu = ur >= 0 ? cells_of(ur) : mine;
-  const Gas<T> c = Gas<T>::make(P);
-  const bool de = NF == 6 && P.dualenergy != 0;
-  const double tend = ctl->tend;
-  double t = ctl->t, dt = ctl->dt;
-  int go = ctl->go, active = ctl->active, k = 0;
-  const bool runnable = ctl->err == 0 && ctl->dump == 0;
-  unsigned err = 0, err_step = 0;   // of this thread: recorded; of the last sweep, not yet exchanged
-  if (tid == 0) s_err = 0u;
+  unsigned err_step = 0;   // this thread's errors of the last sweep, not yet exchanged
   for (int f = 0; f < NF; ++f)
-    for (int i = tid; i < mine; i += NT) qs[f * mine + i] = q[(int64_t)f * n + x0 + i];
-  cl.sync();   // every rank has started before any stores into its shared memory
+    for (int i = tid; i < mine; i += NT) qs[f * mine + i] = q[f * fs + x0 + i];
+  cl.sync();   // every rank is here before any stores into its shared memory
   for (int s = 0;; ++s) {
     const int par = s & 1;
     T* const w = w0 + par * wlen;
     // another step, unless the run has ended (step_begin); the round after
     // the last step only exchanges its errors
-    const bool step = s < nsteps && go != 0 && runnable;
-    active = step ? 1 : (s < nsteps ? 0 : active);
+    const bool step = s < nsteps && L.go != 0 && runnable;
+    L.active = step ? 1 : (s < nsteps ? 0 : L.active);
     T smax = (T)0;
     unsigned e = 0;
     if (step) {
@@ -380,43 +404,89 @@ __global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q
       ge |= mx.err[par][i];
     }
     ge = __reduce_or_sync(0xffffffffu, ge);
-    if (ge >> 16) {   // the last sweep failed: done but not counted, and nothing after it
-      err |= ge >> 16;
-      if (s < nsteps) active = 0;
+    if (ge >> 16) {   // the last sweep failed: nothing after it
+      L.err |= ge >> 16;
+      if (TUBE) ++L.k;
+      if (s < nsteps) L.active = 0;
       break;
     }
-    if (s > 0) ++k;
+    if (s > 0) ++L.k;
     if (!step) break;
     const double gm = (double)warp_max_pos(g);
     unsigned ed = ge & 0xffffu;
-    double d = 0.0;
+    double d = 0.0, t = L.t;
+    int go = L.go;
     if (!ed) d = cfl_dt1(P, gm, ed);
+    if (!ed) update_time(L.tend, t, d, go);
+    if (TUBE && !ed && go && !(t > L.t)) ed |= EVORA_ERR_DT;   // dt below the resolution of t: no progress
     if (ed) {         // hydrostep's errors: no update
-      err |= ed;
-      active = 0;
+      L.err |= ed;
+      L.active = 0;
       break;
     }
-    update_time(tend, t, d, go);
-    dt = d;
+    L.t = t;
+    L.dt = d;
+    L.go = go;
     err_step = 0;
-    tube_sweep<T, NF, NT>(qs, w, mine, P, c, de, dt, err_step);
+    if (mine > 0) tube_sweep<T, NF, NT>(qs, w, mine, P, c, de, d, err_step);
     __syncthreads();
   }
-  if (err && lane == 0) atomicOr(&s_err, err);
   for (int f = 0; f < NF; ++f)
-    for (int i = tid; i < mine; i += NT) q[(int64_t)f * n + x0 + i] = qs[f * mine + i];
-  __syncthreads();
-  if (rank == 0 && tid == 0) {
-    ctl->t = t;
-    ctl->dt = dt;
-    ctl->go = go;
-    ctl->active = active;
-    ctl->k += k;
-    ctl->err |= s_err;
+    for (int i = tid; i < mine; i += NT) q[f * fs + x0 + i] = qs[f * mine + i];
+  cl.sync();   // no rank goes on while its shared memory may be written
+}
+
+template <typename T, int NF, int NT>
+__global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q, GridCtl* ctl, int nsteps, int m) {
+  extern __shared__ __align__(16) unsigned char sraw[];
+  __shared__ LineMax<T, NT> mx;
+  LineRun L{ctl->t, ctl->dt, ctl->tend, ctl->go, ctl->active, 0, 0u};
+  line_steps<T, NF, NT, false>(P, Gas<T>::make(P), NF == 6 && P.dualenergy != 0, q, P.nx, P.nx, m, nsteps,
+                               ctl->err == 0 && ctl->dump == 0, sraw, mx, L);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->t = L.t;
+    ctl->dt = L.dt;
+    ctl->go = L.go;
+    ctl->active = L.active;
+    ctl->k += L.k;
+    ctl->err |= L.err;
     ctl->errnext = 0u;
     ctl->snext[0] = ctl->snext[1] = ctl->snext[2] = 0ull;
   }
-  cl.sync();   // no rank leaves while its shared memory may be written
+}
+
+// The tubes of a small batch, a cluster per tube: a CTA per tube left most SMs
+// idle and the longest tube took its 14 us per step (8192 cells FP32); 8 CTAs
+// take 3.3.  A rank takes at least 64 cells.
+template <typename T, int NF, int NT>
+__global__ void __launch_bounds__(NT) k_tubes_cluster(BatchArgs<T> A) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char sraw[];
+  __shared__ LineMax<T, NT> mx;
+  __shared__ int s_tube;
+  cg::cluster_group cl = cg::this_cluster();
+  const int nr = (int)cl.num_blocks();
+  for (;;) {
+    if (cl.block_rank() == 0 && threadIdx.x == 0) {
+      const int i = atomicAdd(A.head, 1);
+      s_tube = i < A.ntubes ? A.order[i] : -1;
+    }
+    cl.sync();
+    const int tb = *cl.map_shared_rank(&s_tube, 0);
+    cl.sync();   // all have read it
+    if (tb < 0) break;
+    TubeState* ts = A.tubes + tb;
+    if (ts->status != TUBE_RUNNING) continue;
+    const int n = ts->n;
+    const HydroParams P = tube_params(A, n, ts->bt);
+    int m = (n + nr - 1) / nr;
+    if (m < 64) m = 64;
+    while (n % m == 1) ++m;   // every used rank has two cells or more
+    LineRun L{ts->t, ts->dt, ts->tend, 1, 1, 0, 0u};
+    line_steps<T, NF, NT, true>(P, Gas<T>::make(P), P.dualenergy != 0, A.q + ts->offset, A.ntot, n, m,
+                                tube_budget(A, n), true, sraw, mx, L);
+    if (cl.block_rank() == 0 && threadIdx.x == 0) tube_close(A, ts, n, L.t, L.dt, L.k, L.err, L.go);
+  }
 }
 
 }  // namespace EVORA_FNS

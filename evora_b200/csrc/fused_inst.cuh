@@ -489,8 +489,7 @@ void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_
 }
 
 // ---- batched tubes
-template <int NF, int NT>
-void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
+BatchArgs<TT> batch_args(const BatchPlan& pl, void* q) {
   BatchArgs<TT> A;
   A.P = pl.P;
   A.xmin = pl.xmin;
@@ -509,7 +508,56 @@ void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
   A.gscratch = (TT*)pl.gscratch;
   A.nmax = pl.nmax;
   A.cell_updates = pl.cell_updates;
-  k_tubes<TT, NF, NT><<<pl.ctas, NT, pl.smem, st>>>(A);
+  return A;
+}
+
+template <int NF, int NT>
+void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
+  k_tubes<TT, NF, NT><<<pl.ctas, NT, pl.smem, st>>>(batch_args(pl, q));
+}
+
+// A cluster per tube (k_tubes_cluster): 8, 4 or 2 CTAs of 512 threads, as
+// many as let all `running` tubes run at once -- two CTAs per SM in FP32, whose
+// registers and shared memory allow it, one in FP64 -- and 0 where the
+// longest tube does not fit the cluster's shared memory or a CTA per tube
+// fills the SMs.
+template <int NF>
+int cluster_ranks(int running, int nmax, int sms) {
+  const int slots = sms * (sizeof(TT) == 4 ? 2 : 1);
+  const size_t limit = sizeof(TT) == 4 ? kSteps1dSmem / 2 : kSteps1dSmem;
+  for (int r = 8; r >= 2; r /= 2) {
+    const int m = std::max(64, (nmax + r - 1) / r) + 1;
+    if ((long long)running * r <= slots && steps1d_smem(NF, m) <= limit) return r;
+  }
+  return 0;
+}
+
+template <int NF>
+bool cluster_launch(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st) {
+  const int r = cluster_ranks<NF>(running, nmax, sms);
+  if (r == 0) return false;
+  const size_t smem = steps1d_smem(NF, std::max(64, (nmax + r - 1) / r) + 1);
+  auto k = k_tubes_cluster<TT, NF, 512>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(running * r);
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = r;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, batch_args(pl, q));   // errors: cudaGetLastError
+  return true;
+}
+
+bool batch_cluster(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st) {
+  return pl.nf == 5 ? cluster_launch<5>(pl, q, running, nmax, sms, st) : cluster_launch<6>(pl, q, running, nmax, sms, st);
 }
 
 template <int NF, int NT>

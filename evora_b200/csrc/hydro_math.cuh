@@ -456,6 +456,13 @@ __device__ __forceinline__ double mul_rn(double a, double b) {   // a product th
   return a * b;
 #endif
 }
+__device__ __forceinline__ float mul_rn(float a, float b) {
+#if defined(__CUDA_ARCH__)
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
 __device__ __forceinline__ double sq3(double a, double b, double c) { return fma(c, c, fma(b, b, a * a)); }
 
 // q2w with dual energy (comp.f90:26-43, 45-85) in the fast forms: one
@@ -587,7 +594,7 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   const T fk = left ? facl : facr;
   const T ud = w[DIR];
   const T u2 = w[1] * w[1] + w[2] * w[2] + w[3] * w[3];
-  const T e = (T)0.5 * w[0] * u2 + w[4] * c.g1inv;   // total energy
+  const T e = fma((T)0.5 * w[0], u2, mul_rn(w[4], c.g1inv));   // total energy
   const T mu = w[0] * ud;                            // mass flux
   T fl[6], ql[6];
   ql[0] = w[0];
@@ -600,7 +607,7 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   fl[2] = mu * w[2];
   fl[3] = mu * w[3];
   fl[DIR] += w[4];
-  fl[4] = ud * (e + w[4]);
+  fl[4] = mul_rn(ud, e + w[4]);
   T rpg = (T)0;   // 1 / rho^(g-1); 1 / rho^g = rpg / rho
   if (NF == 6) {
     rpg = rcp_fast(pow_fast(w[0], c.g1));
@@ -620,10 +627,13 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   qx[2] = chi * w[2];
   qx[3] = chi * w[3];
   qx[DIR] = chi * sm;
-  qx[4] = chi * (e * ri + (sm - ud) * (sm + w[4] * rcp_fast(fk)));
+  qx[4] = fma(e, ri, mul_rn(sm - ud, fma(w[4], rcp_fast(fk), sm)));
   if (NF == 6) qx[5] = chi * w[4] * (rpg * ri);
 #pragma unroll
-  for (int i = 0; i < NF; ++i) f[i] = fl[i] + sk * (qx[i] - ql[i]);
+  for (int i = 0; i < NF; ++i)
+    // the energy's sums of two products as explicit fmas: left to the compiler,
+    // the kernels of a precision would not all take the same
+    f[i] = i == 4 ? fma(sk, fma(chi, qx[4], -e), fl[4]) : fl[i] + sk * (qx[i] - ql[i]);
 }
 
 // HLL (riemann.f90:47-92) in the fast form, FP64: with the speeds clamped to

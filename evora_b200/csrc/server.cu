@@ -120,6 +120,8 @@ struct evora_server {
   HydroParams P{};
   int precision = EVORA_FP32;
   int flags = 0;
+  int sms = 148;
+  int longest = 0;        // cells of the longest tube in the queue order
   int nf = 5;
   size_t budget = 0, used = 0;
   int steps_per_tick = 64;       // base step count of a round
@@ -496,6 +498,7 @@ int upload_order(evora_server* s) {
   if (!ord.empty())
     CU(cudaMemcpyAsync(s->order, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice, s->tstream));
   s->plan.ntubes = (int)ord.size();
+  s->longest = ord.empty() ? 0 : s->reqs[s->slot_req[ord[0]]].nx;
   s->order_dirty = false;
   return 0;
 }
@@ -605,6 +608,7 @@ int evora_server_create(const evora_params* base, int32_t precision, int32_t fla
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int per_sm = batch_ctas_per_sm(precision, (flags & EVORA_STRICT) != 0, s->nf, nt, pl.smem);
+    s->sms = sms;
     pl.ctas = std::max(1, sms * std::max(1, per_sm));
     if (max_tube_cells > pl.cap) {
       size_t need = (size_t)pl.ctas * (size_t)(s->nf + 5) * (size_t)(max_tube_cells + 4) * s->esize();
@@ -685,7 +689,9 @@ int evora_server_tick(evora_server* s, int32_t* n_active, int32_t* n_pending) {
   if (s->plan.ntubes > 0) {
     if (timed_tubes) CU(cudaEventRecord(s->ev[0], s->tstream));
     CU(cudaMemsetAsync(s->head, 0, sizeof(int), s->tstream));
-    s->launch(s->plan, s->q, s->tstream);
+    if (!batch_cluster_for(s->precision, (s->flags & EVORA_STRICT) != 0, s->plan, s->q, s->plan.ntubes, s->longest,
+                           s->sms, s->tstream))
+      s->launch(s->plan, s->q, s->tstream);
     CU(cudaGetLastError());
     if (timed_tubes) CU(cudaEventRecord(s->ev[1], s->tstream));
   }

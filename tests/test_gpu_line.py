@@ -108,3 +108,53 @@ def test_tubes_strict_bitwise_at_chunk_edges(cuda_device, lengths):
     b.close()
     ref = np.concatenate([w.reshape(-1, 6) for w in want])
     assert np.array_equal(got[:, :5], ref[:, :5])
+
+
+@pytest.mark.parametrize("bt", [1, 2, 3])
+@pytest.mark.parametrize("lengths", [[2, 63, 64, 65, 66, 127, 129], [511, 512, 513, 1025] * 9, [2049, 3000, 8] * 40,
+                                     [5000, 14000]])
+def test_tube_clusters_strict_bitwise(cuda_device, lengths, bt):
+    """Small batches (clusters of 8, 4 and 2 CTAs per tube, and one CTA for the
+    lengths that fit none) against the configured shape and the oracle."""
+    kw = dict(g=5.0 / 3.0, cfl=0.4, boundtype=bt, limiter=1, solver=2, tend=1e9)
+    rng = np.random.default_rng(len(lengths))
+    states = {}
+    for n in set(lengths):
+        o = Oracle(make_params(nx=n, ny=1, nz=1, **kw))
+        q = random_q(o, rng)
+        w = q.copy()
+        o.run(w, 5)
+        states[n] = (q.reshape(-1, 6), w.reshape(-1, 6))
+    q = np.concatenate([states[n][0] for n in lengths])
+    for configured in (False, True):
+        b = ev.Batch(ev.default_params(nx=max(lengths), ny=1, nz=1, **kw), lengths, ev.FP64, ev.STRICT)
+        if configured:
+            b.configure(256, 1)
+        b.set_q(q)
+        assert b.run(max_steps=2) == 0 and b.run(max_steps=3) == 0
+        got = b.get_q()
+        assert all(b.info(i)["k"] == 5 for i in range(0, len(lengths), 7))
+        b.close()
+        assert np.array_equal(got[:, :5], np.concatenate([states[n][1] for n in lengths])[:, :5])
+
+
+def test_tube_clusters_end_and_error(cuda_device):
+    """Tubes of a small batch end at their own times and fail alone."""
+    lengths, q = ev.ic.random_tubes(12, seed=4, nmin=100, nmax=900)
+    p = ev.default_params(nx=max(lengths), ny=1, nz=1, g=5.0 / 3.0, cfl=0.8, boundtype=1, solver=2, tend=0.02)
+    offs = np.concatenate([[0], np.cumsum(lengths)])
+    q[offs[3] + 5, 4] = -1.0
+    res = []
+    for configured in (False, True):
+        b = ev.Batch(p, lengths, ev.FP64, ev.STRICT)
+        if configured:
+            b.configure(256, 1)
+        b.set_tend(2, 0.01)
+        b.set_q(q)
+        b.run()
+        res.append((b.get_q(), [b.info(i) for i in range(12)]))
+        b.close()
+    assert res[0][1] == res[1][1]
+    assert res[0][1][3]["status"] == 2 and res[0][1][3]["k"] == 0 and res[0][1][3]["err"] & 1
+    assert res[0][1][2]["t"] == 0.01 and all(i["status"] == 1 for j, i in enumerate(res[0][1]) if j != 3)
+    assert np.array_equal(res[0][0], res[1][0])
