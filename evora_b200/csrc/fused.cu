@@ -70,28 +70,42 @@ int choose_zc(const HydroParams& P, int precision, int tx, int ty, int minb, int
   return best_zc;
 }
 
-// Rows per warp of the 2D march.  A warp takes R + 2 rows for R of them, and
-// a row takes longer the more warps share the SM: measured (1.0 + 0.032 w) us
-// in FP32 and (1.82 + 0.08 w) us in FP64 with w warps, up to the 16 and 12 that
-// the registers allow.  The R with the shortest sum over the waves of warps;
-// few rows on small grids (64^2: 1), many on large ones (1024^2: 16).
-int choose_rows(const HydroParams& P, int cols, int precision) {
+// Rows per warp of the 2D march, and whether they are unrolled (one or two
+// rows).  Measured us per step with w warps per SM, FP32 / FP64:
+//   R rows in a loop  3.7 + (R + 2) (1.0 + 0.032 w) / 2.5 + (R + 2) (1.82 + 0.08 w),
+//                     up to the 16 / 12 warps that the registers allow
+//   one row           5.4 + 0.23 w / 6.0 + 0.23 w   } up to 20 / 9 warps
+//   two rows          6.7 + 0.19 w / 8.6 + 0.10 w   }
+// The R with the shortest time over the waves of warps: one row on small
+// grids (64^2: 6.8 -> 5.5 / 7.4 -> 6.2 by unrolling), many on large ones (1024^2:
+// 16).
+int choose_rows(const HydroParams& P, int cols, int precision, bool* unrolled) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaGetLastError();
   const bool f32 = precision == EVORA_FP32;
-  const int resident = f32 ? 16 : 12;
-  const double alone = f32 ? 1.0 : 1.82, shared = f32 ? 0.032 : 0.08;
+  const int resident = f32 ? 16 : 12, resident_u = f32 ? 20 : 9;
+  const double base = f32 ? 3.7 : 2.5, alone = f32 ? 1.0 : 1.82, shared = f32 ? 0.032 : 0.08;
   const int64_t strips = (P.nx + cols - 1) / cols;
   double best = 1e300;
   int best_r = 1;
+  *unrolled = false;
   for (int r = 1; r <= 64 && r <= P.ny; ++r) {
     const int64_t per_sm = (strips * ((P.ny + r - 1) / r) + sms - 1) / sms;
     const int64_t full = per_sm / resident, rest = per_sm % resident;
-    const double t = (r + 2) * (full * (alone + shared * resident) + (rest ? alone + shared * rest : 0.0));
+    const double t = base + (r + 2) * (full * (alone + shared * resident) + (rest ? alone + shared * rest : 0.0));
     if (t < best) {
       best = t;
       best_r = r;
+      *unrolled = false;
+    }
+    if (r <= 2 && per_sm <= resident_u) {
+      const double u = r == 1 ? (f32 ? 5.4 : 6.0) + 0.23 * per_sm : (f32 ? 6.7 + 0.19 * per_sm : 8.6 + 0.10 * per_sm);
+      if (u < best) {
+        best = u;
+        best_r = r;
+        *unrolled = true;
+      }
     }
   }
   return best_r;
@@ -109,7 +123,7 @@ void fused_set_tile(FusedPlan* pl, int tile) {
     int64_t b = (P.nx + 127) / 128;
     pl->grid = dim3((unsigned)(b < 1 ? 1 : b), 1, 1);
   } else if (pl->dim == 2) {
-    pl->zc = choose_rows(P, pl->tx, pl->precision);
+    pl->zc = choose_rows(P, pl->tx, pl->precision, &pl->unrolled);
     const int64_t warps = (int64_t)((P.nx + pl->tx - 1) / pl->tx) * ((P.ny + pl->zc - 1) / pl->zc);
     const int per = pl->threads / 32;
     pl->grid = dim3((unsigned)((warps + per - 1) / per), 1, 1);

@@ -35,6 +35,7 @@ struct FusedPlan {
   // writes into ctl->snext (2D and 3D kernels), so that step needs no CFL
   // kernel
   int cfl_fused = 0;
+  bool unrolled = false;   // 2D: the march with its one or two rows (zc) unrolled
   int tail = 0;      // the update's share of the step control (step_tail, fused_kernel.cuh)
   int ranks1d = 0;   // 1D: CTAs of the cluster that runs several steps in one launch (0: the grid does not fit one)
 };

@@ -121,10 +121,11 @@ void launch(const FusedPlan& pl, const void* qin, void* qout, GridCtl* ctl, cuda
   if constexpr (DIM == 1) {
     k_fused1d<TT, NF><<<pl.grid, pl.threads, 0, st>>>(A);
   } else if constexpr (DIM == 2) {
-    if (pl.P.limiter == 1 && pl.P.solver == 2 && pl.P.secondorder)
-      launch_step(pl, k_march2d<TT, NF, true>, pl.threads, 0, st, A);
-    else
-      launch_step(pl, k_march2d<TT, NF, false>, pl.threads, 0, st, A);
+    const bool opt = pl.P.limiter == 1 && pl.P.solver == 2 && pl.P.secondorder;
+    auto k = opt ? k_march2d<TT, NF, true, 0> : k_march2d<TT, NF, false, 0>;
+    if (pl.unrolled && pl.zc == 1) k = opt ? k_march2d<TT, NF, true, 1> : k_march2d<TT, NF, false, 1>;
+    if (pl.unrolled && pl.zc == 2) k = opt ? k_march2d<TT, NF, true, 2> : k_march2d<TT, NF, false, 2>;
+    launch_step(pl, k, pl.threads, 0, st, A);
   } else {
     using C = Tile<I>;
 #if EVORA_PRECISION_F32

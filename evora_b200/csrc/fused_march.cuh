@@ -15,8 +15,8 @@
 // replaces in 2D (fused_tile) has a CTA of 128 or 256 threads go through four
 // barriers for one tile and solves the halo's primitives 1.7 times.  us per
 // step, FP32 / FP64, the tile program with its control kernel -> this:
-// 64^2 8.8 / 11.0 -> 7.1 / 8.4, 512^2 22.7 / 43.2 -> 14.7 / 24.8,
-// 1024^2 64.3 / 156 -> 31.5 / 78.5, 1400^2 119 / 289 -> 60 / 148.
+// 64^2 8.8 / 11.0 -> 5.5 / 6.2, 512^2 22.7 / 43.2 -> 14.7 / 23.2,
+// 1024^2 64.3 / 156 -> 31.7 / 72, 1400^2 119 / 289 -> 55 / 130.
 #pragma once
 
 #include "fused_kernel.cuh"
@@ -29,10 +29,11 @@ constexpr int kMarchWarps = 4;    // warps per CTA
 
 // Warp gw of the grid's strips x chunks (A.zc rows per chunk).  cm: running
 // maxima of |u_d| + a of the written cells.
-template <typename T, int NF, bool OPT>
+// RC > 0: that many rows per warp, the rows unrolled (their chains overlap).
+template <typename T, int NF, bool OPT, int RC = 0>
 __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, unsigned& cerr) {
   const HydroParams& P = A.P;
-  const int nx = P.nx, ny = P.ny, R = A.zc;
+  const int nx = P.nx, ny = P.ny, R = RC > 0 ? RC : A.zc;
   const int lane = threadIdx.x & 31;
   const int nstrips = (nx + kMarchCols - 1) / kMarchCols;
   const int X0 = (gw % nstrips) * kMarchCols, Y0 = (gw / nstrips) * R;
@@ -90,8 +91,11 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
   for (int f = 0; f < 5; ++f) yu[f] = (T)0;
 #pragma unroll
   for (int f = 0; f < NF; ++f) fy[f] = qacc[f] = (T)0;
-  for (int r = Y0 - 1; r <= Y0 + ye; ++r) {
-    const bool inner = r >= Y0 && r < Y0 + ye;
+#pragma unroll (RC > 0 ? RC + 2 : 1)
+  for (int it = 0; it < (RC > 0 ? RC + 2 : ye + 2); ++it) {
+    const int r = Y0 - 1 + it;
+    if (RC > 0 && r > Y0 + ye) break;
+    const bool inner = it >= 1 && (RC == 0 || it <= RC) && r < Y0 + ye;
     T qc[6];
     if (inner) load(r, qc);
     // slopes, predictor and faces of row r
@@ -107,12 +111,12 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
         },
         P, dt2, wv, face);
     // the interface below row r completes row r-1
-    if (r >= Y0) {
+    if (it >= 1) {
       T fn[NF];
       unsigned e = 0;
       riemann_k<T, NF, 2>(yu, face[1][0], fn, solver, c, e);
       if (owned) err |= e;
-      if (r > Y0 && owned) {
+      if (it >= 2 && owned) {
         const int64_t idx = (int64_t)(r - 1) * nx + x;
         T qo[NF];
 #pragma unroll
@@ -184,13 +188,13 @@ __device__ __forceinline__ void march_maxima(GridCtl* ctl, const T* cm, unsigned
 // constants (1024^2 FP32: 43 -> 33 us).  CTAs per SM: FP32 needs 115 registers,
 // so 4; FP64 at 3 (168 registers) or 4 (128, with spills) takes 27 or 30 us at
 // 512^2, 78.5 or 77.6 at 1024^2.
-template <typename T, int NF, bool OPT>
-__global__ void __launch_bounds__(32 * kMarchWarps, sizeof(T) == 4 ? 4 : 3) k_march2d(FusedArgs<T> A) {
+template <typename T, int NF, bool OPT, int RC>
+__global__ void __launch_bounds__(32 * kMarchWarps, RC > 0 ? 2 : (sizeof(T) == 4 ? 4 : 3)) k_march2d(FusedArgs<T> A) {
   __shared__ T red[3][kMarchWarps];
   T cm[3] = {(T)0, (T)0, (T)0};
   unsigned cerr = 0;
   step_head();
-  march2d<T, NF, OPT>(A, blockIdx.x * kMarchWarps + (threadIdx.x >> 5), cm, cerr);
+  march2d<T, NF, OPT, RC>(A, blockIdx.x * kMarchWarps + (threadIdx.x >> 5), cm, cerr);
   if (A.cfl_next) march_maxima(A.ctl, cm, cerr, red);
   step_tail(A);
 }
