@@ -537,7 +537,7 @@ __device__ __forceinline__ void hllc_fast64(const double* wl, const double* wr, 
   const bool pure_right = !pure_left && 0.0 >= sr;
   const bool star = !pure_left && !pure_right;
   const bool left = pure_left || (star && 0.0 < sm);
-  if (!(sl == sl && sr == sr && sm == sm)) err |= EVORA_ERR_HLLC;
+  if (!(sm == sm)) err |= EVORA_ERR_HLLC;   // NaN in sl or sr makes sm NaN
   double w[5];
 #pragma unroll
   for (int i = 0; i < 5; ++i) w[i] = left ? wl[i] : wr[i];
@@ -587,7 +587,7 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   const bool pure_right = !pure_left && (T)0 >= sr;
   const bool star = !pure_left && !pure_right;
   const bool left = pure_left || (star && (T)0 < sm);
-  if (!(sl == sl && sr == sr && sm == sm)) err |= EVORA_ERR_HLLC;
+  if (!(sm == sm)) err |= EVORA_ERR_HLLC;   // NaN in sl or sr makes sm NaN
   const T* w = left ? wl : wr;
   const T ri = left ? ril : rir;
   const T sk = left ? sl : sr;

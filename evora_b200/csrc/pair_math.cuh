@@ -194,8 +194,7 @@ __device__ __forceinline__ void hllc_p(const P2<S>* wl, const P2<S>* wr, P2<S>* 
     star.y = !ply && !pry;
     left.x = plx || (star.x && (S)0 < sm.x);
     left.y = ply || (star.y && (S)0 < sm.y);
-    if (!(sl.x == sl.x && sr.x == sr.x && sm.x == sm.x && sl.y == sl.y && sr.y == sr.y && sm.y == sm.y))
-      err |= EVORA_ERR_HLLC;
+    if (!(sm.x == sm.x && sm.y == sm.y)) err |= EVORA_ERR_HLLC;   // NaN in sl or sr makes sm NaN
   }
   P2<S> w[5];
 #pragma unroll
