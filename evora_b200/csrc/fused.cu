@@ -208,6 +208,8 @@ __global__ void k_from_aos(const double* __restrict__ aos, T* __restrict__ q, in
 // shared memory and written as one run; written by their own threads, at a
 // stride of 48 or 96 bytes, the stores took twice the time of their bytes
 // (256^3 FP32: 398 -> 292 us, FP64 415 -> 307 us; 128^3 with species 158 -> 75).
+// The library's pow and division then bound the FP32 case (FP64 pipe); in the
+// fast forms: 229 us..
 template <typename T>
 __global__ void __launch_bounds__(256) k_to_aos(const T* __restrict__ q, double* __restrict__ aos, int64_t n, int nf,
                                                 double g1, int nq, const double* __restrict__ species) {
@@ -219,9 +221,14 @@ __global__ void __launch_bounds__(256) k_to_aos(const T* __restrict__ q, double*
       load_cell(q, n, nf, i, v);
       if (nf == 5) {
         double m2 = (v[1] * v[1]) + (v[2] * v[2]) + (v[3] * v[3]);
-        double kin = 0.5 * m2 / v[0];
-        double p = g1 * (v[4] - kin);
-        v[5] = p / pow(v[0], g1);
+        if constexpr (sizeof(T) == 4) {   // an FP32 state: a few ulp of FP64 are far below its rounding
+          const double p = g1 * (v[4] - 0.5 * m2 * rcp_fast(v[0]));
+          v[5] = p * rcp_fast(pow_fast(v[0], g1));
+        } else {
+          double kin = 0.5 * m2 / v[0];
+          double p = g1 * (v[4] - kin);
+          v[5] = p / pow(v[0], g1);
+        }
       }
       double* c = cells + (int)threadIdx.x * nq;
 #pragma unroll
