@@ -427,7 +427,9 @@ __device__ __forceinline__ T minmod_fast(T dwl, T dwr) {
 
 // The other limiters (muscl.f90:141-163) in the fast form: the monotonised
 // central one without branches (the central difference has the sign the two
-// others share), van Leer's with the fast reciprocal in FP64.
+// others share; signs are compared, as slope1 does: a product of differences
+// below 1e-19 (FP32) would be flushed and the slope lost), van Leer's with
+// the fast reciprocal in FP64.
 template <typename T>
 __device__ __forceinline__ T slope_fast(T wl, T w, T wr, int limiter) {
   const T dwl = w - wl, dwr = wr - w;
@@ -435,7 +437,7 @@ __device__ __forceinline__ T slope_fast(T wl, T w, T wr, int limiter) {
   if (limiter == 2) {
     const T dwc = (wr - wl) * (T)0.5;
     const T m = fmin(fmin((T)2.0 * fabs(dwl), fabs(dwc)), (T)2.0 * fabs(dwr));
-    return dwl * dwr > (T)0 ? copysign(m, dwl) : (T)0;
+    return (dwl >= (T)0) == (dwr >= (T)0) ? copysign(m, dwl) : (T)0;
   }
   if constexpr (sizeof(T) == 8) {
     const T pro = dwl * dwr;
