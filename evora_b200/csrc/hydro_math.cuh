@@ -613,8 +613,8 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   T rpg = (T)0;   // 1 / rho^(g-1); 1 / rho^g = rpg / rho
   if (NF == 6) {
     rpg = rcp_fast(pow_fast(w[0], c.g1));
-    fl[5] = ud * w[4] * rpg;
-    ql[5] = w[4] * rpg;
+    fl[5] = mul_rn(ud * w[4], rpg);
+    ql[5] = mul_rn(w[4], rpg);
   }
   if (!star) {
 #pragma unroll
@@ -623,19 +623,20 @@ __device__ __forceinline__ void hllc_fast(const T* wl, const T* wr, T* f, const 
   }
   // star state (statex, riemann.f90:241-288)
   const T chi = fk * rcp_fast(sk - sm);           // rho (s - u_d) / (s - sm)
-  T qx[6];
+  T qx[5];
   qx[0] = chi;
   qx[1] = chi * w[1];
   qx[2] = chi * w[2];
   qx[3] = chi * w[3];
   qx[DIR] = chi * sm;
   qx[4] = fma(e, ri, mul_rn(sm - ud, fma(w[4], rcp_fast(fk), sm)));
-  if (NF == 6) qx[5] = chi * w[4] * (rpg * ri);
 #pragma unroll
-  for (int i = 0; i < NF; ++i)
-    // the energy's sums of two products as explicit fmas: left to the compiler,
-    // the kernels of a precision would not all take the same
+  for (int i = 0; i < 5; ++i)
+    // the energy's (and the entropy's) sums of two products as explicit fmas:
+    // left to the compiler, the kernels of a precision would not all take the
+    // same
     f[i] = i == 4 ? fma(sk, fma(chi, qx[4], -e), fl[4]) : fl[i] + sk * (qx[i] - ql[i]);
+  if (NF == 6) f[5] = fma(sk, fma(chi * w[4], rpg * ri, -ql[5]), fl[5]);
 }
 
 // HLL (riemann.f90:47-92) in the fast form, FP64: with the speeds clamped to
