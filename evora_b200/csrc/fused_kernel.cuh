@@ -1032,7 +1032,10 @@ __device__ __forceinline__ void hydro_control(const HydroParams& P, GridCtl* ctl
 // Start of an update that may be launched while the previous one still runs
 // (programmatic dependent launch): lets the next one start being launched and
 // waits until the previous one is complete.  Without that launch attribute
-// both are no-ops.
+// both are no-ops.  The state is written while CTAs of this launch may already
+// be resident, so they read it with ordinary loads only: __ldg is for data
+// that does not change while a kernel runs, and its cache may still hold what
+// an earlier update read from the same buffer.
 __device__ __forceinline__ void step_head() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   asm volatile("griddepcontrol.wait;\n" ::: "memory");

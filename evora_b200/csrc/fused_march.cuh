@@ -68,7 +68,7 @@ __device__ __forceinline__ void march2d(const FusedArgs<T>& A, int gw, T* cm, un
   auto load = [&](int y, T* qv) {
     const T* p = A.qin + row(y);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) qv[f] = ld(p + f * n);
+    for (int f = 0; f < NF; ++f) qv[f] = p[f * n];   // coherent loads: step_head
   };
   auto convert = [&](T* qv, T* wv) {
     prim_k(qv, wv, c, P, de, err);
