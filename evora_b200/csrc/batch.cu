@@ -475,12 +475,19 @@ int evora_batch_run(evora_batch* b, int32_t max_steps, int32_t sync) {
   if (it == b->graphs.end()) {
     // capture: reset the queue head, then the persistent kernel
     b->plan.budget = budget;
-    cudaGraph_t g;
+    cudaGraph_t g = nullptr;
+    cudaGetLastError();   // an older error is not this launch's
     CU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
     if (!b->clusters || !batch_cluster_for(b->precision, b->strict, b->plan, b->q, b->ntubes, b->nmax, b->sms, b->stream))
       b->launch(b->plan, b->q, b->stream);
-    CU(cudaStreamEndCapture(b->stream, &g));
+    const cudaError_t refused = cudaGetLastError();
+    cudaError_t ended = cudaStreamEndCapture(b->stream, &g);
+    if (refused != cudaSuccess || ended != cudaSuccess) {   // no graph without the tubes' kernel is kept
+      if (g) cudaGraphDestroy(g);
+      set_cuda_error(refused != cudaSuccess ? refused : ended, "evora_batch_run: launch");
+      return EVORA_ERR_CUDA;
+    }
     cudaGraphExec_t ex;
     cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);

@@ -410,14 +410,29 @@ void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) {
   else k_cfl_soa<6><<<(int)blocks, 256, 0, st>>>(pl.P, (const TT*)q, pl.n, ctl);
 }
 
+// ---- dynamic shared memory of the kernels below
+// A launch is refused when it asks for more than its kernel's limit, and the
+// limit belongs to the kernel, not to a plan: batches, servers and grids of
+// other lengths share it, in other threads too.  So it is always the most that
+// the device gives (its opt-in size less the kernel's static memory), set when
+// a plan is made and never to a plan's own size.
+template <class Kernel>
+void allow_smem(Kernel k) {
+  int dev = 0, most = 0;
+  cudaFuncAttributes a;
+  if (cudaGetDevice(&dev) == cudaSuccess && cudaFuncGetAttributes(&a, k) == cudaSuccess &&
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess)
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+  cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  cudaGetLastError();
+}
+
 // ---- 1D grids: several steps in one launch
-constexpr size_t kSteps1dSmem = 220 * 1024;
+constexpr size_t kSteps1dSmem = 220 * 1024;   // + 6 KB static: within allow_smem's limit
 size_t steps1d_smem(int nf, int m) { return ((size_t)10 * (m + 4) + (size_t)nf * m) * sizeof(TT); }
 
 template <int NF, int NT>
 void steps1d_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int ranks, size_t smem, cudaStream_t st) {
-  cudaFuncSetAttribute(k_steps1d<TT, NF, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (ranks > 8) cudaFuncSetAttribute(k_steps1d<TT, NF, NT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(ranks);
   cfg->blockDim = dim3(NT);
@@ -437,6 +452,13 @@ void steps1d_launch(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, int 
   cudaLaunchAttribute at;
   steps1d_config<NF, NT>(&cfg, &at, pl.ranks1d, steps1d_smem(NF, m), st);
   cudaLaunchKernelEx(&cfg, k_steps1d<TT, NF, NT>, pl.P, (TT*)q, ctl, nsteps, m);   // errors: cudaGetLastError
+}
+
+template <int NF>
+void steps1d_allow() {
+  allow_smem(k_steps1d<TT, NF, 256>);
+  allow_smem(k_steps1d<TT, NF, 512>);
+  cudaFuncSetAttribute(k_steps1d<TT, NF, 512>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
 template <int NF>
@@ -465,6 +487,8 @@ bool steps1d_wide(int m) {   // whether this device schedules clusters of 16 suc
 // (FP32) cells.
 int steps1d_plan(const FusedPlan& pl) {
   if (pl.dim != 1) return 0;
+  if (pl.nf == 5) steps1d_allow<5>();
+  else steps1d_allow<6>();
   auto per_rank = [&](int r) { return (int)((pl.n + r - 1) / r); };
   auto fits = [&](int r) {
     const int m = per_rank(r);
@@ -538,9 +562,6 @@ bool cluster_launch(const BatchPlan& pl, void* q, int running, int nmax, int sms
   const int r = cluster_ranks<NF>(running, nmax, sms);
   if (r == 0) return false;
   const size_t smem = steps1d_smem(NF, std::max(64, (nmax + r - 1) / r) + 1);
-  auto k = k_tubes_cluster<TT, NF, 512>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(running * r);
   cfg.blockDim = dim3(512);
@@ -553,7 +574,7 @@ bool cluster_launch(const BatchPlan& pl, void* q, int running, int nmax, int sms
   at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k, batch_args(pl, q));   // errors: cudaGetLastError
+  cudaLaunchKernelEx(&cfg, k_tubes_cluster<TT, NF, 512>, batch_args(pl, q));   // errors: cudaGetLastError
   return true;
 }
 
@@ -566,9 +587,8 @@ BatchLaunch batch_pick_one(BatchPlan* pl) {
   pl->threads = NT;
   pl->smem = ((size_t)NF * pl->cap + 5 * ((size_t)pl->cap + 4)) * sizeof(TT);
   pl->capw = std::max(pl->cap, (int)(pl->smem / (5 * sizeof(TT))) - 4);
-  auto k = k_tubes<TT, NF, NT>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl->smem);
-  cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  allow_smem(k_tubes<TT, NF, NT>);
+  allow_smem(k_tubes_cluster<TT, NF, 512>);
   return &batch_launch<NF, NT>;
 }
 
@@ -587,7 +607,7 @@ BatchLaunch batch_pick(int nf, int threads, BatchPlan* pl) {
 template <int NF, int NT>
 int max_ctas_one(size_t smem) {
   int nb = 0;
-  cudaFuncSetAttribute(k_tubes<TT, NF, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(k_tubes<TT, NF, NT>);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tubes<TT, NF, NT>, NT, smem);
   return nb;
 }
