@@ -63,6 +63,7 @@ struct BatchPlan {
   int threads = 256;   // NT
   int ctas = 1;        // persistent grid
   size_t smem = 0;
+  int clusters[4] = {0, 0, 0, 0};   // clusters of 2^i CTAs that run at once (k_tubes_cluster)
 };
 
 #define EVORA_DECLARE_BATCH_NS(ns)                                                          \

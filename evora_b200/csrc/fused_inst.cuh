@@ -541,39 +541,83 @@ void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
   k_tubes<TT, NF, NT><<<pl.ctas, NT, pl.smem, st>>>(batch_args(pl, q));
 }
 
-// A cluster per tube (k_tubes_cluster): 8, 4 or 2 CTAs of 512 threads, as
-// many as let all `running` tubes run at once -- two CTAs per SM in FP32, whose
-// registers and shared memory allow it, one in FP64 -- and 0 where the
-// longest tube does not fit the cluster's shared memory or a CTA per tube
-// fills the SMs.
+// Cells per rank of the longest tube, as k_tubes_cluster splits it (at most).
+int cluster_cells(int nmax, int ranks) { return std::max(64, (nmax + ranks - 1) / ranks) + 1; }
+
+// CTAs per tube (k_tubes_cluster, 512 threads each): 2, 4 or 8, or 0 for a CTA
+// per tube (k_tubes), by the shortest estimated step of the longest tube.
+// pl.clusters has the clusters of each size that run at once (74, 33 and 15 of
+// 2, 4 and 8 CTAs: one CTA fits an SM, and the SMs of a GPC that do not make up
+// a whole cluster stay idle); more tubes than that wait for one another.
+// us per step of equal tubes, measured, FP32 / FP64:
+//     cells       CTA          2            4            8 CTAs, all at once
+//        60   1.1 / 1.4    1.8 / 2.0    1.8 / 2.0    1.8 / 2.1
+//       150   1.8 / 2.3    1.8 / 2.0    1.8 / 2.0    1.8 / 2.1
+//       500   1.9 / 3.1    2.0 / 2.5    1.9 / 2.3    1.9 / 2.2
+//      1000   2.9 / 5.0    2.5 / 3.5    2.0 / 2.6    2.0 / 2.5
+//      2500   5.8 / 10.5   3.8 / 6.1    2.8 / 4.1    2.2 / 2.8
+//      8000  20.2 / 36.6    - / -       5.2 / -      3.7 / 5.6
+// and twice or three times that in two or three turns.  With every tube a
+// cluster up to two CTAs per SM, the rule before, 148 FP32 tubes of 1000 cells
+// took 4.9 (now 2.9), 37 of 2500 6.5 (3.8), 24 of 60 3.5 (1.1).
 template <int NF>
-int cluster_ranks(int running, int nmax, int sms) {
-  const int slots = sms * (sizeof(TT) == 4 ? 2 : 1);
-  const size_t limit = sizeof(TT) == 4 ? kSteps1dSmem / 2 : kSteps1dSmem;
-  for (int r = 8; r >= 2; r /= 2) {
-    const int m = std::max(64, (nmax + r - 1) / r) + 1;
-    if ((long long)running * r <= slots && steps1d_smem(NF, m) <= limit) return r;
+int cluster_ranks(const BatchPlan& pl, int running, int nmax, int sms) {
+  if (running > sms) return 0;   // not even a CTA per tube at once: measured with fewer
+  constexpr bool f32 = sizeof(TT) == 4;
+  const double cta = f32 ? std::max(nmax <= 120 ? 1.1 : 1.75, 0.95 + 1.9e-3 * nmax)
+                         : std::max(nmax <= 120 ? 1.4 : 2.3, 1.2 + 3.75e-3 * nmax);
+  double best = cta;
+  int ranks = 0;
+  for (int i = 1; i <= 3; ++i) {
+    const int m = cluster_cells(nmax, 1 << i), at_once = pl.clusters[i];
+    if (at_once < 1 || steps1d_smem(NF, m) > kSteps1dSmem) continue;
+    const double t = ((running + at_once - 1) / at_once) * (f32 ? 1.75 + 1.78e-3 * m : 1.9 + 3.5e-3 * m);
+    if (t < best) {
+      best = t;
+      ranks = 1 << i;
+    }
   }
-  return 0;
+  return ranks;
+}
+
+template <int NF>
+void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int tubes, int ranks, size_t smem,
+                    cudaStream_t st) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(tubes * ranks);
+  cfg->blockDim = dim3(512);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = st;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = ranks;
+  at->val.clusterDim.y = 1;
+  at->val.clusterDim.z = 1;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+}
+
+// The clusters that run at once, with the most shared memory a launch asks for.
+template <int NF>
+void cluster_plan(BatchPlan* pl) {
+  allow_smem(k_tubes_cluster<TT, NF, 512>);
+  for (int i = 1; i <= 3; ++i) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    cluster_config<NF>(&cfg, &at, 1, 1 << i, kSteps1dSmem, nullptr);
+    int count = 0;
+    if (cudaOccupancyMaxActiveClusters(&count, k_tubes_cluster<TT, NF, 512>, &cfg) != cudaSuccess) count = 0;
+    pl->clusters[i] = count;
+  }
+  cudaGetLastError();
 }
 
 template <int NF>
 bool cluster_launch(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st) {
-  const int r = cluster_ranks<NF>(running, nmax, sms);
+  const int r = cluster_ranks<NF>(pl, running, nmax, sms);
   if (r == 0) return false;
-  const size_t smem = steps1d_smem(NF, std::max(64, (nmax + r - 1) / r) + 1);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(running * r);
-  cfg.blockDim = dim3(512);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
+  cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = r;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cluster_config<NF>(&cfg, &at, running, r, steps1d_smem(NF, cluster_cells(nmax, r)), st);
   cudaLaunchKernelEx(&cfg, k_tubes_cluster<TT, NF, 512>, batch_args(pl, q));   // errors: cudaGetLastError
   return true;
 }
@@ -588,7 +632,7 @@ BatchLaunch batch_pick_one(BatchPlan* pl) {
   pl->smem = ((size_t)NF * pl->cap + 5 * ((size_t)pl->cap + 4)) * sizeof(TT);
   pl->capw = std::max(pl->cap, (int)(pl->smem / (5 * sizeof(TT))) - 4);
   allow_smem(k_tubes<TT, NF, NT>);
-  allow_smem(k_tubes_cluster<TT, NF, 512>);
+  cluster_plan<NF>(pl);
   return &batch_launch<NF, NT>;
 }
 

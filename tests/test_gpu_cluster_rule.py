@@ -1,0 +1,41 @@
+"""The rule that gives each tube of a small batch a cluster of CTAs: only
+where that is no slower than a CTA per tube."""
+import numpy as np
+import pytest
+
+import evora_b200 as ev
+
+pytestmark = pytest.mark.gpu
+
+
+def us_per_step(lengths, q, precision, threads):
+    import torch
+    p = ev.default_params(nx=max(lengths), ny=1, nz=1, g=5.0 / 3.0, cfl=0.4, boundtype=2, tend=1e9)
+    stream = torch.cuda.Stream()
+    with ev.Batch(p, lengths, precision) as b:
+        b.set_stream(stream)
+        if threads:
+            b.configure(threads, 1)
+        b.set_q(q)
+        b.run(max_steps=200)
+        times = []
+        for _ in range(7):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record(stream)
+            b.run(max_steps=200, sync=False)
+            e1.record(stream)
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+    return 5.0 * min(times)
+
+
+# more tubes than clusters of 2, 4 or 8 CTAs that run at once, and tubes too
+# short to be shared; 25 %: the spread of single launches and of the rule's
+# model of them
+@pytest.mark.parametrize("count,n,precision,threads", [
+    (148, 1000, ev.FP32, 512), (100, 2500, ev.FP32, 512), (24, 60, ev.FP32, 128), (18, 60, ev.FP64, 128),
+    (33, 400, ev.FP32, 256), (74, 2500, ev.FP64, 512), (16, 5000, ev.FP64, 512)])
+def test_clusters_are_not_slower(cuda_device, count, n, precision, threads):
+    lengths, q = ev.ic.random_tubes(count, seed=n, nmin=n, nmax=n)
+    chosen = us_per_step(lengths, q, precision, None)
+    assert chosen <= 1.25 * us_per_step(lengths, q, precision, threads)
