@@ -147,10 +147,13 @@ int configure(evora_batch* b, int threads, int cap) {
 // of 64 to 8000 cells (G cell-updates/s, FP32 / FP64):
 //   128 threads up to 700 cells (512 cells: 67.8 / 34.5, with 256 60.1 / 28.0),
 //   256 up to 1500 (1024 cells: 69.9 / 33.3, with 512 54.8 / 26.9),
-//   512 above (4096 cells: 64.7 / 30.9, with 256 41.2 / 23.2);
-// as many CTAs per SM as the registers hold, or one that can take any tube in
-// FP64.  With no more than two tubes per SM the longest ones decide, so a tube gets all
-// warps that it has rounds of 30 cells for.
+//   512 above, one CTA per SM, which is what its registers (97 and more) allow
+//   and whose shared memory takes a tube of 5756 (FP32) or 2876 cells: 3000
+//   cells FP32 64.9; with the memory of half an SM, the rule before, 42.6;
+//   with 256 threads 56.1 (4096 tubes of 128-4096: 59.6, 38.7, 17.6);
+// with 128 and 256 as many CTAs per SM as the registers hold.  With no more
+// than two tubes per SM the longest ones decide, so a tube gets all warps that
+// it has rounds of 30 cells for.
 int configure_default(evora_batch* b) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -161,7 +164,7 @@ int configure_default(evora_batch* b) {
     return configure(b, b->nmax > 480 ? 512 : (b->nmax > 240 ? 256 : 128), cap_for(b, 1));
   if (len <= 700.0) return configure(b, 128, cap_for(b, f32 ? 6 : 4));
   if (len <= 1500.0) return configure(b, 256, cap_for(b, f32 ? 3 : 2));
-  return configure(b, 512, cap_for(b, f32 ? 2 : 1));
+  return configure(b, 512, cap_for(b, 1));
 }
 
 int upload_order(evora_batch* b) {
