@@ -98,13 +98,15 @@ double work_length(const evora_batch* b) {
   return n3 / n2;
 }
 
-// cap: tubes up to this length are staged in shared memory.  A single CTA
-// of 512 threads per SM becomes one of 768 where long tubes do most of the
-// work: at 4096 cells 66.9 against 62.1 G cell-updates/s (FP32) and 30.9
-// against 29.4 (FP64), at 8000 cells 48.6 against 40.0; at 2048 cells it
-// loses 1 to 5 %.
+// Whether a single CTA per SM has 768 threads rather than 512 by default:
+// where long tubes do most of the work (at 4096 cells 66.9 against 62.1 G
+// cell-updates/s in FP32 and 30.9 against 29.4 in FP64, at 8000 cells 48.6
+// against 40.0; at 2048 cells it loses 1 to 5 %).  Six fields need more
+// registers than 768 threads have.
+bool wide_pays(const evora_batch* b) { return b->nf == 5 && work_length(b) > 2600.0; }
+
+// cap: tubes up to this length are staged in shared memory.
 int configure(evora_batch* b, int threads, int cap) {
-  if (threads == 512 && b->nf == 5 && cap >= cap_for(b, 1) && work_length(b) > 2600.0) threads = 768;
   drop_graphs(b);
   BatchPlan& pl = b->plan;
   pl.P = b->P;
@@ -160,11 +162,12 @@ int configure_default(evora_batch* b) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const double len = work_length(b);
   const bool f32 = b->precision == EVORA_FP32;
+  const int one = wide_pays(b) ? 768 : 512;   // of a single CTA per SM
   if (b->ntubes <= 2 * sms)
-    return configure(b, b->nmax > 480 ? 512 : (b->nmax > 240 ? 256 : 128), cap_for(b, 1));
+    return configure(b, b->nmax > 480 ? one : (b->nmax > 240 ? 256 : 128), cap_for(b, 1));
   if (len <= 700.0) return configure(b, 128, cap_for(b, f32 ? 6 : 4));
   if (len <= 1500.0) return configure(b, 256, cap_for(b, f32 ? 3 : 2));
-  return configure(b, 512, cap_for(b, 1));
+  return configure(b, one, cap_for(b, 1));
 }
 
 int upload_order(evora_batch* b) {
@@ -535,8 +538,8 @@ int evora_batch_steps_done(evora_batch* b, int64_t* cell_updates) {
 }
 
 int evora_batch_configure(evora_batch* b, int32_t threads, int32_t ctas_per_sm) {
-  if (!b || (threads != 128 && threads != 256 && threads != 512) || ctas_per_sm < 1 || ctas_per_sm > 8)
-    return EVORA_ERR_ARG;
+  if (!b || ctas_per_sm < 1 || ctas_per_sm > 8) return EVORA_ERR_ARG;
+  if (threads != 128 && threads != 256 && threads != 512 && !(threads == 768 && b->nf == 5)) return EVORA_ERR_ARG;
   CU(cudaStreamSynchronize(b->stream));
   b->clusters = false;
   return configure(b, threads, cap_for(b, ctas_per_sm));
@@ -567,41 +570,51 @@ int evora_batch_autotune(evora_batch* b, int32_t steps, int32_t* threads_out, in
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
-  const int cand_threads[3] = {128, 256, 512};
-  const int cand_ctas[3] = {1, 2, 3};
-  float best = 1e30f;
+  // One trial of the configured shape, or of clusters (false: they do not
+  // serve this batch).
+  auto trial = [&](bool clusters, float* ms) -> int {
+    *ms = 1e30f;
+    b->plan.budget = steps;
+    b->plan.steps_per_cell = (double)steps * b->ntubes / (double)b->ntot;
+    CU(cudaEventRecord(e0, b->stream));
+    cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
+    const bool ran = !clusters || batch_cluster_for(b->precision, b->strict, b->plan, b->q, b->ntubes, b->nmax,
+                                                    b->sms, b->stream);
+    if (!clusters) b->launch(b->plan, b->q, b->stream);
+    CU(cudaEventRecord(e1, b->stream));
+    CU(cudaEventSynchronize(e1));
+    CU(cudaGetLastError());
+    b->plan.steps_per_cell = 0.0;
+    if (ran) CU(cudaEventElapsedTime(ms, e0, e1));
+    CU(cudaMemcpyAsync(b->q, save_q, qbytes, cudaMemcpyDeviceToDevice, b->stream));
+    CU(cudaMemcpyAsync(b->tubes, save_t, sizeof(TubeState) * b->ntubes, cudaMemcpyDeviceToDevice, b->stream));
+    return 0;
+  };
+  const int cand_threads[4] = {128, 256, 512, 768};
+  float best = 1e30f, ms = 0.f;
   int bt = 256, bc = 2;
-  for (int ti = 0; ti < 3; ++ti)
-    for (int ci = 0; ci < 3; ++ci) {
-      if (configure(b, cand_threads[ti], cap_for(b, cand_ctas[ci]))) continue;
-      b->plan.budget = steps;
-      b->plan.steps_per_cell = (double)steps * b->ntubes / (double)b->ntot;
-      CU(cudaEventRecord(e0, b->stream));
-      cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
-      b->launch(b->plan, b->q, b->stream);
-      CU(cudaEventRecord(e1, b->stream));
-      CU(cudaEventSynchronize(e1));
-      CU(cudaGetLastError());
-      b->plan.steps_per_cell = 0.0;
-      float ms = 0.f;
-      CU(cudaEventElapsedTime(&ms, e0, e1));
+  for (int ti = 0; ti < (wide_pays(b) ? 4 : 3); ++ti)
+    for (int ctas = 1; ctas <= (cand_threads[ti] == 768 ? 1 : 3); ++ctas) {
+      if (configure(b, cand_threads[ti], cap_for(b, ctas))) continue;
+      int rc = trial(false, &ms);
+      if (rc) return rc;
       if (ms < best) {
         best = ms;
         bt = cand_threads[ti];
-        bc = cand_ctas[ci];
+        bc = ctas;
       }
-      CU(cudaMemcpyAsync(b->q, save_q, qbytes, cudaMemcpyDeviceToDevice, b->stream));
-      CU(cudaMemcpyAsync(b->tubes, save_t, sizeof(TubeState) * b->ntubes, cudaMemcpyDeviceToDevice, b->stream));
     }
+  int rc = trial(true, &ms);
+  if (rc) return rc;
+  b->clusters = ms < best;
   CU(cudaMemcpyAsync(b->cell_updates, &cu0, sizeof cu0, cudaMemcpyHostToDevice, b->stream));
   CU(cudaStreamSynchronize(b->stream));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(save_q);
   cudaFree(save_t);
-  b->clusters = false;
-  if (threads_out) *threads_out = bt;
-  if (ctas_out) *ctas_out = bc;
+  if (threads_out) *threads_out = b->clusters ? 512 : bt;
+  if (ctas_out) *ctas_out = b->clusters ? 1 : bc;
   return configure(b, bt, cap_for(b, bc));
 }
 

@@ -535,11 +535,16 @@ int evora_batch_info(evora_batch* b, int32_t tube, double* t, double* dt, int32_
                      int32_t* status);
 /* Total cell-updates done by the batch so far. */
 int evora_batch_steps_done(evora_batch* b, int64_t* cell_updates);
-/* Threads per CTA (128, 256, 512) and CTAs per SM the shared-memory staging
- * is sized for (tubes longer than that capacity run from global memory). */
+/* A CTA per tube: threads per CTA (128, 256, 512; 768 with 5 fields) and CTAs
+ * per SM the shared-memory staging is sized for (tubes longer than that
+ * capacity run from global memory).  Without this call the shape follows from
+ * the lengths, and the tubes of a small batch share clusters of CTAs. */
 int evora_batch_configure(evora_batch* b, int32_t threads, int32_t ctas_per_sm);
-/* Autotuner: times every (threads, CTAs per SM) candidate for `steps` steps
- * on the batch's own state (restored after each trial) and keeps the fastest. */
+/* Autotuner: times every (threads, CTAs per SM) candidate, and clusters where
+ * the batch is small, for `steps` steps of a tube of mean length on the
+ * batch's own state (restored after each trial) and keeps the fastest.
+ * Reports its threads and CTAs per SM (512 and 1 for clusters, which
+ * evora_batch_configure does not choose). */
 int evora_batch_autotune(evora_batch* b, int32_t steps, int32_t* threads, int32_t* ctas_per_sm);
 
 /* ------------------------------------------------------------- serving -- */
