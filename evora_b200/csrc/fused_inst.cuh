@@ -596,9 +596,14 @@ void cluster_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int tubes,
   cfg->numAttrs = 1;
 }
 
-// The clusters that run at once, with the most shared memory a launch asks for.
+// The clusters that run at once, with the most shared memory a launch asks
+// for.  A batch of more tubes than SMs never asks; loading the kernel for it
+// would cost its first creation some 5 ms.
 template <int NF>
 void cluster_plan(BatchPlan* pl) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (pl->ntubes > sms) return;
   allow_smem(k_tubes_cluster<TT, NF, 512>);
   for (int i = 1; i <= 3; ++i) {
     cudaLaunchConfig_t cfg;
