@@ -1344,7 +1344,7 @@ int evora_multigrid_step(evora_multigrid* m, int32_t nsteps, int32_t sync) {
   for (evora_grid* g : m->grids) {
     if (nsteps & 1) g->cur ^= 1;
     g->cfl_fresh = g->plan.cfl_fused != 0;
-    g->launches += (1LL + m->has3 + m->has2) * nsteps + 1;
+    g->launches += (1LL + m->has3 + m->has2) * nsteps + (nsteps + 31) / 32;   // a closing control per chunk
     m->cell_updates += (long long)nsteps * ncells(g);
   }
   if (sync) CU(cudaStreamSynchronize(m->stream));
