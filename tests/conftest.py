@@ -16,6 +16,21 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: longer CPU test")
 
 
+# modules whose every test compares with the translated reference
+NEEDS_REFERENCE = ("test_gpu_noncie_hydro",)
+
+
+def pytest_collection_modifyitems(items):
+    """As the other tests of the translated reference: skipped where it is not
+    built."""
+    from oracle import ref_oracle
+    if not ref_oracle.available():
+        skip = pytest.mark.skip(reason="translated reference not built")
+        for item in items:
+            if item.module.__name__ in NEEDS_REFERENCE:
+                item.add_marker(skip)
+
+
 @pytest.fixture(scope="session")
 def cuda_device():
     """The CUDA device for GPU tests.  Fails (does not skip) without one: a
