@@ -173,7 +173,7 @@ void fused_plan_free(FusedPlan* pl) {
 
 void fused_cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) { pl.cfl(pl, q, ctl, st); }
 
-void fused_steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
+void fused_steps1d(FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
   if (pl.precision == EVORA_FP32) f32::steps1d(pl, q, ctl, nsteps, st);
   else if (pl.strict) f64s::steps1d(pl, q, ctl, nsteps, st);
   else f64::steps1d(pl, q, ctl, nsteps, st);

@@ -38,6 +38,7 @@ struct FusedPlan {
   bool unrolled = false;   // 2D: the march with its one or two rows (zc) unrolled
   int tail = 0;      // the update's share of the step control (step_tail, fused_kernel.cuh)
   int ranks1d = 0;   // 1D: CTAs of the cluster that runs several steps in one launch (0: the grid does not fit one)
+  bool allowed1d = false;   // its kernels' launch limits are set
 };
 
 // Chooses tiles and the kernel instantiation; allocates small scratch.
@@ -57,7 +58,7 @@ void fused_update(const FusedPlan& plan, const void* qin, void* qout, GridCtl* c
 
 // 1D grids without physics after the update, plan.ranks1d > 0: `nsteps`
 // steps of the state q, in place, in one launch.
-void fused_steps1d(const FusedPlan& plan, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);
+void fused_steps1d(FusedPlan& plan, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);
 
 // Layout conversions between the reference q(6, nx, ny, nz) (FP64) and the
 // resident SoA state.  Without the entropy field, q(6) is written as
@@ -136,7 +137,7 @@ double march_time(int precision, int sms, int resident, double ctas, int zc);
   MultiLaunch multi_pick(int nf, MultiShape* s);                                             \
   void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st);                \
   int steps1d_plan(const FusedPlan& pl);                                                     \
-  void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);      \
+  void steps1d(FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st);      \
   }
 EVORA_DECLARE_FUSED_NS(f64)
 EVORA_DECLARE_FUSED_NS(f64s)

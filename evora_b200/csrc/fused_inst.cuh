@@ -414,8 +414,8 @@ void cfl(const FusedPlan& pl, const void* q, GridCtl* ctl, cudaStream_t st) {
 // A launch is refused when it asks for more than its kernel's limit, and the
 // limit belongs to the kernel, not to a plan: batches, servers and grids of
 // other lengths share it, in other threads too.  So it is always the most that
-// the device gives (its opt-in size less the kernel's static memory), set when
-// a plan is made and never to a plan's own size.
+// the device gives (its opt-in size less the kernel's static memory), set once
+// by each plan and never to a plan's own size.
 template <class Kernel>
 void allow_smem(Kernel k) {
   int dev = 0, most = 0;
@@ -465,6 +465,7 @@ template <int NF>
 bool steps1d_wide(int m) {   // whether this device schedules clusters of 16 such CTAs
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
+  steps1d_allow<NF>();
   steps1d_config<NF, 512>(&cfg, &at, 16, steps1d_smem(NF, m), nullptr);
   int count = 0;
   const bool ok = cudaOccupancyMaxActiveClusters(&count, k_steps1d<TT, NF, 512>, &cfg) == cudaSuccess;
@@ -487,8 +488,6 @@ bool steps1d_wide(int m) {   // whether this device schedules clusters of 16 suc
 // (FP32) cells.
 int steps1d_plan(const FusedPlan& pl) {
   if (pl.dim != 1) return 0;
-  if (pl.nf == 5) steps1d_allow<5>();
-  else steps1d_allow<6>();
   auto per_rank = [&](int r) { return (int)((pl.n + r - 1) / r); };
   auto fits = [&](int r) {
     const int m = per_rank(r);
@@ -501,7 +500,12 @@ int steps1d_plan(const FusedPlan& pl) {
   return fits(r) ? r : 0;
 }
 
-void steps1d(const FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
+void steps1d(FusedPlan& pl, void* q, GridCtl* ctl, int nsteps, cudaStream_t st) {
+  if (!pl.allowed1d) {   // at a grid's first step: it loads the kernels (15 ms the first time)
+    if (pl.nf == 5) steps1d_allow<5>();
+    else steps1d_allow<6>();
+    pl.allowed1d = true;
+  }
   // warps for one round of 30 cells each, as far as 16 of them go
   const int m = (int)((pl.n + pl.ranks1d - 1) / pl.ranks1d);
   if (pl.nf == 5) {
