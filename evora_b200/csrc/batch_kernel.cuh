@@ -17,8 +17,9 @@
 //   phase 2  each warp updates 30 consecutive cells at a time (muscl.f90:
 //            194-215): a lane per cell and interface, face states and fluxes
 //            passed on by shuffles (tube_sweep).
-// Bound: instruction issue (57 % of the issue slots at 16 warps per SM, 4 %
-// of HBM).  A lane per interface solves every interface once (1.07 times, with
+// Bound: instruction issue (64 % of the issue slots in FP32, 61 % in FP64, at
+// 16 warps per SM; 374 and 673 instructions per cell-update; no HBM traffic to
+// speak of).  A lane per interface solves every interface once (1.07 times, with
 // the 2 of 32 lanes that only feed their neighbours); a contiguous segment of
 // cells per thread, as this kernel first had, solved it (n / NT + 1) / (n /
 // NT) times and read w at strides that met in the banks.  4096 tubes of
@@ -455,9 +456,10 @@ __global__ void __launch_bounds__(NT) k_steps1d(HydroParams P, T* __restrict__ q
   }
 }
 
-// The tubes of a small batch, a cluster per tube: a CTA per tube left most SMs
-// idle and the longest tube took its 14 us per step (8192 cells FP32); 8 CTAs
-// take 3.3.  A rank takes at least 64 cells.
+// The tubes of a small batch, a cluster per tube: a CTA per tube leaves most SMs
+// idle and the longest tube takes its 20 us per step (8000 cells FP32); 8 CTAs
+// take 3.7.  A rank takes at least 64 cells.  By size and count: cluster_ranks
+// (fused_inst.cuh).
 template <typename T, int NF, int NT>
 __global__ void __launch_bounds__(NT) k_tubes_cluster(BatchArgs<T> A) {
   namespace cg = cooperative_groups;

@@ -209,7 +209,7 @@ __global__ void k_from_aos(const double* __restrict__ aos, T* __restrict__ q, in
 // stride of 48 or 96 bytes, the stores took twice the time of their bytes
 // (256^3 FP32: 398 -> 292 us, FP64 415 -> 307 us; 128^3 with species 158 -> 75).
 // The library's pow and division then bound the FP32 case (FP64 pipe); in the
-// fast forms: 229 us..
+// fast forms: 229 us.
 template <typename T>
 __global__ void __launch_bounds__(256) k_to_aos(const T* __restrict__ q, double* __restrict__ aos, int64_t n, int nf,
                                                 double g1, int nq, const double* __restrict__ species) {

@@ -30,7 +30,9 @@
 //
 // The same source compiles for a host emulation (EVORA_HOST_EMU) in which the
 // threads of a CTA are std::threads meeting at a std::barrier, so the tile
-// logic can be checked against the CPU oracle without a GPU.
+// logic can be checked against the CPU oracle without a GPU.  The kernels run
+// it for 3D grids only: 2D ones have the march (fused_march.cuh), and fused_tile's
+// 2D form is left for the host emulation.
 #pragma once
 
 #include <type_traits>
@@ -221,7 +223,7 @@ struct FusedSmem {
   // three-barrier march of FP64 tiles with 5 fields: the next plane's
   // conserved state (with halo), copied asynchronously while a plane is
   // computed (with 6 fields three CTAs would not fit an SM)
-  T raw[NF][!DQ && NF == 5 ? RY * RX : 1];
+  T raw[NF][(!DQ || kHostEmu) && NF == 5 ? RY * RX : 1];
 };
 
 // Whether the shared-memory layout of a march carries dq.
@@ -483,7 +485,7 @@ __device__ __forceinline__ void fused_tile(const FusedArgs<T>& A, FusedSmem<T, N
   // A in two halves for the three-barrier march: each thread copies its halo
   // cells of plane z into sm.raw, and a plane later converts the same cells
   // (waiting for its own copies only).  256^3 FP64: 2.07 -> 1.99 ms per launch.
-  constexpr bool kStaged = DIM == 3 && !PIPE && NF == 5 && sizeof(T) == 8 && !kHostEmu;
+  constexpr bool kStaged = DIM == 3 && !PIPE && NF == 5 && sizeof(T) == 8;
   auto stage_plane = [&](int z) {
     bool zflip = false;
     const int mz = ghost_map(z, nz, P.boundtype, 2, zflip);

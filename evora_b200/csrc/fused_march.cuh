@@ -11,7 +11,7 @@
 //
 // Bound: instruction issue on large grids, the latency of the row's dependent
 // chain on small ones, where the rows per warp (R) are chosen so that the
-// warps fill the SMs (march_rows, fused_inst.cuh).  The tile program this
+// warps fill the SMs (choose_rows, fused.cu).  The tile program this
 // replaces in 2D (fused_tile) has a CTA of 128 or 256 threads go through four
 // barriers for one tile and solves the halo's primitives 1.7 times.  us per
 // step, FP32 / FP64, the tile program with its control kernel -> this:

@@ -91,8 +91,9 @@ struct evora_grid {
 };
 
 // A batch of resident 2D and 3D grids stepped together: per step one control
-// kernel (every grid's hydrostep, updatetime), one persistent update launch
-// over the tiles of all grids, one closing control kernel.
+// kernel (every grid's previous step's end, hydrostep, updatetime), then side
+// by side a persistent update launch over the 3D members' tiles and one over
+// the 2D members' strips; a closing control kernel per call or graph.
 struct evora_multigrid {
   int precision = EVORA_FP64;
   int flags = 0;

@@ -386,8 +386,8 @@ class Grid:
 
 class MultiGrid:
     """Resident 2D and 3D grids of uneven sizes advanced together: per step
-    one control kernel, one persistent update launch over the tiles of all
-    member grids, one closing control kernel (evora_multigrid_*)."""
+    one control kernel and a persistent update launch for the 3D members'
+    tiles and one for the 2D members' strips (evora_multigrid_*)."""
 
     def __init__(self, precision: int = FP32, flags: int = 0, stream=None):
         h = ctypes.c_void_p()

@@ -509,8 +509,8 @@ int evora_grid_timing_split(evora_grid* g, double* cfl_ms, double* update_ms, do
  * its own grid, with its own length n[i], time, step size and end time, all
  * sharing the options of *p (solver, limiter, boundtype, secondorder, g,
  * cfl, xmin/xmax, tstart, tend).  One persistent kernel launch advances every
- * unfinished tube; each CTA stages a whole tube in shared memory and runs its
- * steps there.  Tubes are independent: a tube's result does not depend on the
+ * unfinished tube; a CTA, or in small batches a cluster of CTAs, stages a whole
+ * tube in shared memory and runs its steps there.  Tubes are independent: a tube's result does not depend on the
  * others (bit for bit), and a tube that raises an error stops alone. */
 typedef struct evora_batch evora_batch;
 
