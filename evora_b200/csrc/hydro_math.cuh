@@ -425,6 +425,19 @@ __device__ __forceinline__ T minmod_fast(T dwl, T dwr) {
   return dwl * dwr > (T)0 ? copysign(m, dwl) : (T)0;
 }
 
+// Whether two numbers have the same sign (a zero counts either way here: the
+// slope beside it is zero).  FP32 compares the sign bits, one integer
+// instruction less (100 x 96 x 128 moncen, HLLC: 110.4 -> 105.3 us per step);
+// FP64 kernels have the integer pipe busier (60 x 50 x 40: 33.9, by bits 34.3).
+__device__ __forceinline__ bool same_sign(float a, float b) {
+#if defined(__CUDA_ARCH__)
+  return (__float_as_int(a) ^ __float_as_int(b)) >= 0;
+#else
+  return std::signbit(a) == std::signbit(b);
+#endif
+}
+__device__ __forceinline__ bool same_sign(double a, double b) { return (a >= 0.0) == (b >= 0.0); }
+
 // The other limiters (muscl.f90:141-163) in the fast form: the monotonised
 // central one without branches (the central difference has the sign the two
 // others share; signs are compared, as slope1 does: a product of differences
@@ -437,7 +450,7 @@ __device__ __forceinline__ T slope_fast(T wl, T w, T wr, int limiter) {
   if (limiter == 2) {
     const T dwc = (wr - wl) * (T)0.5;
     const T m = fmin(fmin((T)2.0 * fabs(dwl), fabs(dwc)), (T)2.0 * fabs(dwr));
-    return (dwl >= (T)0) == (dwr >= (T)0) ? copysign(m, dwl) : (T)0;
+    return same_sign(dwl, dwr) ? copysign(m, dwl) : (T)0;
   }
   if constexpr (sizeof(T) == 8) {
     const T pro = dwl * dwr;
