@@ -47,7 +47,8 @@ struct evora_batch {
   BatchLaunch launch = nullptr;
   std::map<int, cudaGraphExec_t> graphs;
   bool order_dirty = true;
-  bool clusters = true;    // the default shape: a cluster per tube where that pays (batch_cluster_for)
+  bool clusters = true;    // the default shape: a cluster per tube where that pays (launch_clusters)
+  std::vector<int> queue;  // the tubes in queue order
   int sms = 148;
 };
 
@@ -176,8 +177,25 @@ int upload_order(evora_batch* b) {
   std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return b->work[a] > b->work[c]; });
   CU(cudaMemcpyAsync(b->order, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice, b->stream));
   CU(cudaStreamSynchronize(b->stream));
+  b->queue = std::move(ord);
   b->order_dirty = false;
   return 0;
+}
+
+// Enqueues the plan's launch by clusters of CTAs, if they serve this batch.
+bool launch_clusters(evora_batch* b) {
+  if (b->ntubes > b->sms) return false;
+  const BatchPlan& pl = b->plan;
+  std::vector<int> n(b->ntubes);
+  std::vector<double> steps(b->ntubes);   // to the tubes' ends as their work has it
+  for (int i = 0; i < b->ntubes; ++i) {
+    const int t = b->queue[i];
+    n[i] = b->n[t];
+    steps[i] = pl.steps_per_cell > 0.0 ? n[i] : (pl.budget >= kBatchToTheEnd ? b->work[t] / n[i] : 1.0);
+  }
+  const int ranks = batch_cluster_ranks_for(b->precision, b->strict, pl, n.data(), steps.data(), b->ntubes, b->sms);
+  if (ranks) batch_cluster_for(b->precision, b->strict, b->plan, b->q, b->ntubes, b->nmax, ranks, b->stream);
+  return ranks != 0;
 }
 
 template <typename T>
@@ -231,10 +249,18 @@ int evora::batch_ctas_per_sm(int precision, int strict, int nf, int threads, siz
   return strict ? f64s::batch_max_ctas_per_sm(nf, threads, smem) : f64::batch_max_ctas_per_sm(nf, threads, smem);
 }
 
-bool evora::batch_cluster_for(int precision, int strict, const BatchPlan& pl, void* q, int running, int nmax, int sms,
-                              cudaStream_t st) {
-  if (precision == EVORA_FP32) return f32::batch_cluster(pl, q, running, nmax, sms, st);
-  return strict ? f64s::batch_cluster(pl, q, running, nmax, sms, st) : f64::batch_cluster(pl, q, running, nmax, sms, st);
+int evora::batch_cluster_ranks_for(int precision, int strict, const BatchPlan& pl, const int* n, const double* steps,
+                                   int running, int sms) {
+  if (precision == EVORA_FP32) return f32::batch_cluster_ranks(pl, n, steps, running, sms);
+  return strict ? f64s::batch_cluster_ranks(pl, n, steps, running, sms)
+                : f64::batch_cluster_ranks(pl, n, steps, running, sms);
+}
+
+void evora::batch_cluster_for(int precision, int strict, const BatchPlan& pl, void* q, int running, int nmax,
+                              int ranks, cudaStream_t st) {
+  if (precision == EVORA_FP32) f32::batch_cluster(pl, q, running, nmax, ranks, st);
+  else if (strict) f64s::batch_cluster(pl, q, running, nmax, ranks, st);
+  else f64::batch_cluster(pl, q, running, nmax, ranks, st);
 }
 
 namespace {
@@ -476,7 +502,7 @@ int evora_batch_run(evora_batch* b, int32_t max_steps, int32_t sync) {
     if (rc) return rc;
   }
   // "to completion" is bounded too: at most 2^24 steps per tube per launch
-  const int budget = max_steps <= 0 ? (1 << 24) : max_steps;
+  const int budget = max_steps <= 0 ? kBatchToTheEnd : max_steps;
   auto it = b->graphs.find(budget);
   if (it == b->graphs.end()) {
     // capture: reset the queue head, then the persistent kernel
@@ -485,8 +511,7 @@ int evora_batch_run(evora_batch* b, int32_t max_steps, int32_t sync) {
     cudaGetLastError();   // an older error is not this launch's
     CU(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
-    if (!b->clusters || !batch_cluster_for(b->precision, b->strict, b->plan, b->q, b->ntubes, b->nmax, b->sms, b->stream))
-      b->launch(b->plan, b->q, b->stream);
+    if (!b->clusters || !launch_clusters(b)) b->launch(b->plan, b->q, b->stream);
     const cudaError_t refused = cudaGetLastError();
     cudaError_t ended = cudaStreamEndCapture(b->stream, &g);
     if (refused != cudaSuccess || ended != cudaSuccess) {   // no graph without the tubes' kernel is kept
@@ -578,8 +603,7 @@ int evora_batch_autotune(evora_batch* b, int32_t steps, int32_t* threads_out, in
     b->plan.steps_per_cell = (double)steps * b->ntubes / (double)b->ntot;
     CU(cudaEventRecord(e0, b->stream));
     cudaMemsetAsync(b->head, 0, sizeof(int), b->stream);
-    const bool ran = !clusters || batch_cluster_for(b->precision, b->strict, b->plan, b->q, b->ntubes, b->nmax,
-                                                    b->sms, b->stream);
+    const bool ran = !clusters || launch_clusters(b);
     if (!clusters) b->launch(b->plan, b->q, b->stream);
     CU(cudaEventRecord(e1, b->stream));
     CU(cudaEventSynchronize(e1));

@@ -40,6 +40,8 @@ struct BatchArgs {
   unsigned long long* cell_updates;  // running total
 };
 
+constexpr int kBatchToTheEnd = 1 << 24;   // the budget of a launch to the tubes' end times
+
 struct BatchPlan;
 typedef void (*BatchLaunch)(const BatchPlan& pl, void* q, cudaStream_t st);
 
@@ -71,8 +73,10 @@ struct BatchPlan {
   /* configures launch for nf fields and `threads` per CTA; sets plan->smem from cap */     \
   BatchLaunch batch_pick(int nf, int threads, BatchPlan* plan);                             \
   int batch_max_ctas_per_sm(int nf, int threads, size_t smem);                              \
-  /* launches a cluster of CTAs per tube where that serves `running` tubes, else false */   \
-  bool batch_cluster(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st);  \
+  /* CTAs of the cluster that each of the running tubes (n[i] cells, about steps[i] */      \
+  /* steps, in queue order) takes; 0: a CTA per tube (the launch of batch_pick) */            \
+  int batch_cluster_ranks(const BatchPlan& pl, const int* n, const double* steps, int running, int sms); \
+  void batch_cluster(const BatchPlan& pl, void* q, int running, int nmax, int ranks, cudaStream_t st);  \
   }
 EVORA_DECLARE_BATCH_NS(f64)
 EVORA_DECLARE_BATCH_NS(f64s)
@@ -87,7 +91,9 @@ void tube_to_aos(const void* q, double* aos, bool f32, long long ntot, long long
 // Instantiation dispatch by precision.
 BatchLaunch batch_pick_for(int precision, int strict, int nf, int threads, BatchPlan* pl);
 int batch_ctas_per_sm(int precision, int strict, int nf, int threads, size_t smem);
-bool batch_cluster_for(int precision, int strict, const BatchPlan& pl, void* q, int running, int nmax, int sms,
+int batch_cluster_ranks_for(int precision, int strict, const BatchPlan& pl, const int* n, const double* steps,
+                            int running, int sms);
+void batch_cluster_for(int precision, int strict, const BatchPlan& pl, void* q, int running, int nmax, int ranks,
                        cudaStream_t st);
 
 }  // namespace evora

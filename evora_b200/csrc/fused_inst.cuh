@@ -7,6 +7,8 @@
 
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+
 #include "batch_kernel.cuh"
 #include "conduction.h"
 #include "fused.h"
@@ -548,11 +550,21 @@ void batch_launch(const BatchPlan& pl, void* q, cudaStream_t st) {
 // Cells per rank of the longest tube, as k_tubes_cluster splits it (at most).
 int cluster_cells(int nmax, int ranks) { return std::max(64, (nmax + ranks - 1) / ranks) + 1; }
 
+// Estimated us per step of a tube of n cells by a CTA, and by ranks of m cells.
+double cta_us(int n) {
+  return sizeof(TT) == 4 ? std::max(n <= 120 ? 1.1 : 1.75, 0.95 + 1.9e-3 * n)
+                         : std::max(n <= 120 ? 1.4 : 2.3, 1.2 + 3.75e-3 * n);
+}
+double cluster_us(int m) { return sizeof(TT) == 4 ? 1.75 + 1.78e-3 * m : 1.9 + 3.5e-3 * m; }
+
 // CTAs per tube (k_tubes_cluster, 512 threads each): 2, 4 or 8, or 0 for a CTA
-// per tube (k_tubes), by the shortest estimated step of the longest tube.
+// per tube (k_tubes), by the shortest estimated time of the launch.
 // pl.clusters has the clusters of each size that run at once (74, 33 and 15 of
 // 2, 4 and 8 CTAs: one CTA fits an SM, and the SMs of a GPC that do not make up
-// a whole cluster stay idle); more tubes than that wait for one another.
+// a whole cluster stay idle); more tubes than that wait for one another, so the
+// queue is played through: each tube goes to the cluster that is free first.
+// n, steps: the running tubes' lengths and steps in the launch (their relation
+// is enough), in queue order.
 // us per step of equal tubes, measured, FP32 / FP64:
 //     cells       CTA          2            4            8 CTAs, all at once
 //        60   1.1 / 1.4    1.8 / 2.0    1.8 / 2.0    1.8 / 2.1
@@ -565,20 +577,24 @@ int cluster_cells(int nmax, int ranks) { return std::max(64, (nmax + ranks - 1) 
 // cluster up to two CTAs per SM, the rule before, 148 FP32 tubes of 1000 cells
 // took 4.9 (now 2.9), 37 of 2500 6.5 (3.8), 24 of 60 3.5 (1.1).
 template <int NF>
-int cluster_ranks(const BatchPlan& pl, int running, int nmax, int sms) {
-  if (running > sms) return 0;   // not even a CTA per tube at once: measured with fewer
-  constexpr bool f32 = sizeof(TT) == 4;
-  const double cta = f32 ? std::max(nmax <= 120 ? 1.1 : 1.75, 0.95 + 1.9e-3 * nmax)
-                         : std::max(nmax <= 120 ? 1.4 : 2.3, 1.2 + 3.75e-3 * nmax);
-  double best = cta;
-  int ranks = 0;
-  for (int i = 1; i <= 3; ++i) {
-    const int m = cluster_cells(nmax, 1 << i), at_once = pl.clusters[i];
-    if (at_once < 1 || steps1d_smem(NF, m) > kSteps1dSmem) continue;
-    const double t = ((running + at_once - 1) / at_once) * (f32 ? 1.75 + 1.78e-3 * m : 1.9 + 3.5e-3 * m);
+int cluster_ranks(const BatchPlan& pl, const int* n, const double* steps, int running, int sms) {
+  if (running < 1 || running > sms) return 0;   // not even a CTA per tube at once: measured with fewer
+  double best = 0.0;
+  int nmax = 0, ranks = 0;
+  for (int i = 0; i < running; ++i) {
+    best = std::max(best, steps[i] * cta_us(n[i]));
+    nmax = std::max(nmax, n[i]);
+  }
+  for (int e = 1; e <= 3; ++e) {
+    double busy[128] = {};   // until when each cluster is
+    const int at_once = std::min(pl.clusters[e], 128);
+    if (at_once < 1 || steps1d_smem(NF, cluster_cells(nmax, 1 << e)) > kSteps1dSmem) continue;
+    for (int i = 0; i < running; ++i)
+      *std::min_element(busy, busy + at_once) += steps[i] * cluster_us(cluster_cells(n[i], 1 << e));
+    const double t = *std::max_element(busy, busy + at_once);
     if (t < best) {
       best = t;
-      ranks = 1 << i;
+      ranks = 1 << e;
     }
   }
   return ranks;
@@ -621,18 +637,20 @@ void cluster_plan(BatchPlan* pl) {
 }
 
 template <int NF>
-bool cluster_launch(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st) {
-  const int r = cluster_ranks<NF>(pl, running, nmax, sms);
-  if (r == 0) return false;
+void cluster_launch(const BatchPlan& pl, void* q, int running, int nmax, int ranks, cudaStream_t st) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
-  cluster_config<NF>(&cfg, &at, running, r, steps1d_smem(NF, cluster_cells(nmax, r)), st);
+  cluster_config<NF>(&cfg, &at, running, ranks, steps1d_smem(NF, cluster_cells(nmax, ranks)), st);
   cudaLaunchKernelEx(&cfg, k_tubes_cluster<TT, NF, 512>, batch_args(pl, q));   // errors: cudaGetLastError
-  return true;
 }
 
-bool batch_cluster(const BatchPlan& pl, void* q, int running, int nmax, int sms, cudaStream_t st) {
-  return pl.nf == 5 ? cluster_launch<5>(pl, q, running, nmax, sms, st) : cluster_launch<6>(pl, q, running, nmax, sms, st);
+int batch_cluster_ranks(const BatchPlan& pl, const int* n, const double* steps, int running, int sms) {
+  return pl.nf == 5 ? cluster_ranks<5>(pl, n, steps, running, sms) : cluster_ranks<6>(pl, n, steps, running, sms);
+}
+
+void batch_cluster(const BatchPlan& pl, void* q, int running, int nmax, int ranks, cudaStream_t st) {
+  if (pl.nf == 5) cluster_launch<5>(pl, q, running, nmax, ranks, st);
+  else cluster_launch<6>(pl, q, running, nmax, ranks, st);
 }
 
 template <int NF, int NT>

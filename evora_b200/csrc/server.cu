@@ -122,6 +122,7 @@ struct evora_server {
   int flags = 0;
   int sms = 148;
   int longest = 0;        // cells of the longest tube in the queue order
+  int ranks = 0;          // CTAs of the cluster that each tube takes (0: a CTA per tube)
   int nf = 5;
   size_t budget = 0, used = 0;
   int steps_per_tick = 64;       // base step count of a round
@@ -498,7 +499,15 @@ int upload_order(evora_server* s) {
   if (!ord.empty())
     CU(cudaMemcpyAsync(s->order, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice, s->tstream));
   s->plan.ntubes = (int)ord.size();
-  s->longest = ord.empty() ? 0 : s->reqs[s->slot_req[ord[0]]].nx;
+  std::vector<int> lengths;
+  std::vector<double> steps;   // of a round (tube_budget)
+  for (int i : ord) {
+    lengths.push_back(s->reqs[s->slot_req[i]].nx);
+    steps.push_back((double)std::min<long long>(s->plan.budget, std::max(1LL, s->plan.quantum / lengths.back())));
+  }
+  s->longest = ord.empty() ? 0 : lengths[0];
+  s->ranks = batch_cluster_ranks_for(s->precision, (s->flags & EVORA_STRICT) != 0, s->plan, lengths.data(),
+                                     steps.data(), (int)lengths.size(), s->sms);
   s->order_dirty = false;
   return 0;
 }
@@ -689,8 +698,10 @@ int evora_server_tick(evora_server* s, int32_t* n_active, int32_t* n_pending) {
   if (s->plan.ntubes > 0) {
     if (timed_tubes) CU(cudaEventRecord(s->ev[0], s->tstream));
     CU(cudaMemsetAsync(s->head, 0, sizeof(int), s->tstream));
-    if (!batch_cluster_for(s->precision, (s->flags & EVORA_STRICT) != 0, s->plan, s->q, s->plan.ntubes, s->longest,
-                           s->sms, s->tstream))
+    if (s->ranks)
+      batch_cluster_for(s->precision, (s->flags & EVORA_STRICT) != 0, s->plan, s->q, s->plan.ntubes, s->longest,
+                        s->ranks, s->tstream);
+    else
       s->launch(s->plan, s->q, s->tstream);
     CU(cudaGetLastError());
     if (timed_tubes) CU(cudaEventRecord(s->ev[1], s->tstream));

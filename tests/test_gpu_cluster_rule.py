@@ -39,3 +39,30 @@ def test_clusters_are_not_slower(cuda_device, count, n, precision, threads):
     lengths, q = ev.ic.random_tubes(count, seed=n, nmin=n, nmax=n)
     chosen = us_per_step(lengths, q, precision, None)
     assert chosen <= 1.25 * us_per_step(lengths, q, precision, threads)
+
+
+@pytest.mark.parametrize("count,lo,hi", [(50, 100, 6000), (74, 30, 1500)])
+def test_clusters_serve_mixed_lengths(cuda_device, count, lo, hi):
+    """More tubes than clusters that run at once: the short ones wait for the
+    long ones, which still end sooner than with a CTA each."""
+    import torch
+    lengths, q = ev.ic.random_tubes(count, seed=hi + count, nmin=lo, nmax=hi)
+    p = ev.default_params(nx=hi, ny=1, nz=1, g=5.0 / 3.0, cfl=0.4, boundtype=1, tend=0.005)
+    best = []
+    for threads in (None, 512):
+        stream = torch.cuda.Stream()
+        with ev.Batch(p, lengths, ev.FP32) as b:
+            b.set_stream(stream)
+            if threads:
+                b.configure(threads, 1)
+            times = []
+            for _ in range(4):
+                b.set_q(q)
+                e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                e0.record(stream)
+                b.run(sync=False)
+                e1.record(stream)
+                torch.cuda.synchronize()
+                times.append(e0.elapsed_time(e1))
+        best.append(min(times))
+    assert best[0] <= best[1]
